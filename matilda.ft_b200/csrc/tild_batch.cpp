@@ -176,8 +176,18 @@ void Batch::buildGroup(Group &G)
         e.nfg = nfg;
         e.int_tile_max = b->ppHost.int_tile_max;
         e.dq = b->ppHost.dchan_charge;
-        e.Lx = fft_batch_lines(BS_XFWD, b->geom, nfg);
-        e.Lxi = fft_batch_lines(BS_XINV, b->geom, nfg);
+        e.two = b->twoStage ? 1 : 0;
+        if (e.two) {
+            const long long cols = (long long)e.g.nz * e.g.hp;
+            e.Lx = fft2_xfwd_lines(e.g, e.lx, (nd + 1) / 2);
+            e.Lxi = fft2_xinv_lines(e.g, e.lx, nfg);
+            e.cby = fft2_col_bits(e.ly, cols, nd);
+            e.cbyi = fft2_col_bits(e.ly, cols, 2 * nfg);
+            e.cbz = kspace2_col_bits(e.g, e.lz, nd);
+        } else {
+            e.Lx = fft_batch_lines(BS_XFWD, b->geom, nfg);
+            e.Lxi = fft_batch_lines(BS_XINV, b->geom, nfg);
+        }
         e.txz = G.txz;
         e.ks_npots = (int)b->potentials.size();
         e.X0 = b->dX[0];
@@ -203,18 +213,24 @@ void Batch::buildGroup(Group &G)
         deposit_batch_shape(e, deterministic, &blocks, &threads, &smem, &cap);
         e.dep_cap = cap;
     }
-    // every stage's prefix table of CTA counts, its widest CTA and largest shared memory
-    std::vector<int> pre((size_t)(BS_COUNT + 1) * (R + 1), 0);
-    for (int s = 0; s <= BS_COUNT; s++) {
-        int *ps = pre.data() + (size_t)s * (R + 1);
-        BatchLaunch &bl = G.launches[s];
+    // every stage's prefix table of CTA counts, its widest CTA and largest shared memory; the
+    // second set of tables deals the transforms of the replicas with two-stage lines
+    std::vector<int> pre((size_t)(2 * BS_COUNT) * (R + 1), 0);
+    auto transform = [](int s) { return s != BS_DEPOSIT && s != BS_GATHER && s != BS_INTEGRATE; };
+    for (int t = 0; t < 2 * BS_COUNT; t++) {
+        const int s = t % BS_COUNT, two = t / BS_COUNT;
+        int *ps = pre.data() + (size_t)t * (R + 1);
+        BatchLaunch &bl = two ? G.launches2[s] : G.launches[s];
         bl.threads = 0;
         bl.smem = 0;
         for (int r = 0; r < R; r++) {
             int blocks = 0, threads = 256, cap = 0;
             size_t smem = 0;
-            if (s == BS_COUNT) zero_batch_shape(h[r], deterministic, &blocks);
-            else if (s == BS_DEPOSIT) deposit_batch_shape(h[r], deterministic, &blocks, &threads, &smem, &cap);
+            if (transform(s) ? h[r].two != two : two != 0) {
+                ps[r + 1] = ps[r];
+                continue;
+            }
+            if (s == BS_DEPOSIT) deposit_batch_shape(h[r], deterministic, &blocks, &threads, &smem, &cap);
             else if (s == BS_GATHER || s == BS_INTEGRATE) particles_batch_shape(s, h[r], &blocks, &threads, &smem);
             else fft_batch_shape(s, h[r], &blocks, &threads, &smem);
             ps[r + 1] = ps[r] + blocks;
@@ -227,15 +243,23 @@ void Batch::buildGroup(Group &G)
     batch_ck(cudaMalloc(&G.dPre, sizeof(int) * pre.size()), "cudaMalloc");
     batch_ck(cudaMemcpy(G.dReps, h.data(), sizeof(BatchRep) * R, cudaMemcpyHostToDevice), "table upload");
     batch_ck(cudaMemcpy(G.dPre, pre.data(), sizeof(int) * pre.size(), cudaMemcpyHostToDevice), "table upload");
-    for (int s = 0; s <= BS_COUNT; s++) G.launches[s].pre = G.dPre + (size_t)s * (R + 1);
-    // the step: zero, deposit, x/y forward, k-space, y/x inverse, gather, integrate, tick
+    for (int s = 0; s < BS_COUNT; s++) {
+        G.launches[s].pre = G.dPre + (size_t)s * (R + 1);
+        G.launches2[s].pre = G.dPre + (size_t)(BS_COUNT + s) * (R + 1);
+    }
+    // the step: deposit, x/y forward, k-space, y/x inverse, gather, integrate, tick
     const cudaStream_t st = G.stream;
     cudaGraph_t gr;
     batch_ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-    cudaError_t e = launch_zero_batch(G.dReps, R, G.launches[BS_COUNT], deterministic, st);
-    if (e == cudaSuccess) e = launch_deposit_batch(G.dReps, R, G.launches[BS_DEPOSIT], order, nd, deterministic, st);
+    cudaError_t e = launch_deposit_batch(G.dReps, R, G.launches[BS_DEPOSIT], order, nd, deterministic, st);
     for (int s : {BS_XFWD, BS_YFWD, BS_KSPACE, BS_YINV, BS_XINV})
-        if (e == cudaSuccess) e = launch_fft_batch(s, G.dReps, R, G.launches[s], deterministic, G.txz, st);
+    {
+        if (e == cudaSuccess && G.launches[s].blocks)
+            e = launch_fft_batch(s, G.dReps, R, G.launches[s], deterministic, G.txz, st);
+        if (e == cudaSuccess && G.launches2[s].blocks)
+            e = s == BS_KSPACE ? launch_kspace2_batch(G.dReps, R, G.launches2[s], nd, st)
+                               : launch_fft2_batch(s, G.dReps, R, G.launches2[s], deterministic, st);
+    }
     for (int s : {BS_GATHER, BS_INTEGRATE})
         if (e == cudaSuccess) e = launch_particles_batch(s, G.dReps, R, G.launches[s], order, nfg, extra, st);
     if (e == cudaSuccess) e = launch_batch_tick(G.dReps, R, st);

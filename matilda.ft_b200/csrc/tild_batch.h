@@ -5,11 +5,12 @@
 // A batch holds boxes (endBox processed) that share the kernels' compile-time settings:
 // 3-D, the same spline order, one or two density fields, one or two force groups, the
 // same deterministic mode, the tile gather over paired records.  Their sizes, grids,
-// potentials, tiles and integrators may all differ.  Every step stage -- zeroing the
-// deposit targets, the deposit, the five transform passes, the tile gather, the integrator
-// pass, the step counters -- is ONE launch whose CTAs are dealt over the replicas' work by
+// potentials, tiles and integrators may all differ.  Every step stage -- the
+// deposit, the five transform passes, the tile gather, the integrator
+// pass, the step counters -- is ONE launch (a transform pass two, where only some replicas'
+// lines run in two register stages) whose CTAs are dealt over the replicas' work by
 // a prefix table of CTA counts; each replica's geometry, FFT plans, tile lists, record
-// layout, TMA descriptors and arrays sit in a device table.  The ten launches of a step are
+// layout, TMA descriptors and arrays sit in a device table.  The launches of a step are
 // captured once in a CUDA graph.  Every sort_interval steps each replica's spatial re-sort
 // runs as a branch of one more graph.
 //
@@ -41,7 +42,8 @@ private:
         int txz = 0;
         BatchRep *dReps = nullptr;
         int *dPre = nullptr;                     // the stages' prefix tables, (R + 1) ints each
-        BatchLaunch launches[BS_COUNT + 1];      // + the zeroing of the deposit targets
+        BatchLaunch launches[BS_COUNT];          // every replica, or the mixed-radix ones' transforms
+        BatchLaunch launches2[BS_COUNT];         // transforms of the replicas with two-stage lines
         cudaGraphExec_t gStep = nullptr, gSort = nullptr;
     };
     void build();

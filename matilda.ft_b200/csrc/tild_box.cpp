@@ -1088,6 +1088,9 @@ void Box::buildPlan()
     g.M = (long long)g.nx * g.ny * g.nz;
     if (g.M >= (1ll << 31)) fail(TILD_ERR_UNSUPPORTED, "grids of 2^31 points or more");
     g.hstride = (long long)g.nz * g.ny * g.hp;
+    g.dhp = make_fastdiv((unsigned)g.hp);
+    g.dny = make_fastdiv((unsigned)g.ny);
+    g.dnxh = make_fastdiv((unsigned)g.nxh);
     for (int j = 0; j < 3; j++) {
         g.dxf[j] = (float)dx[j];
         g.dlo[j] = (float)(dx[j] - (double)g.dxf[j]);
@@ -1230,23 +1233,28 @@ void Box::allocDevice()
     if (rngCompat) dRng = dalloc<unsigned char>(N * rng_state_bytes());
     const int nd = std::max(1, (int)dfields.size()), nfg = std::max(1, (int)fgroups.size());
     const int npair = (nd + 1) / 2;
-    if (deterministic) dDepFix = dalloc<unsigned long long>((size_t)2 * npair * g.M);
-    else dDep = dalloc<float2>((size_t)npair * g.M);
+    // the deposit target starts at zero; every x forward pass clears what it has read
+    if (deterministic) {
+        dDepFix = dalloc<unsigned long long>((size_t)2 * npair * g.M);
+        ck(cudaMemsetAsync(dDepFix, 0, sizeof(unsigned long long) * 2 * npair * g.M, stream), "zero deposit");
+    } else {
+        dDep = dalloc<float2>((size_t)npair * g.M);
+        ck(cudaMemsetAsync(dDep, 0, sizeof(float2) * npair * g.M, stream), "zero deposit");
+    }
     dH = dalloc<float2>((size_t)nd * g.hstride);
     dHg = dalloc<float2>((size_t)3 * nfg * g.hstride);
-    dTw = dalloc<float2>((size_t)g.nx + g.ny + g.nz);
-    build_fft_line(g.nx, lx, dTw);
-    build_fft_line(g.ny, ly, dTw + g.nx);
-    build_fft_line(g.nz, lz, dTw + g.nx + g.ny);
+    dTw = dalloc<float2>(3 * ((size_t)g.nx + g.ny + g.nz));
+    build_fft_line(g.nx, ksHost.twopi_over_L[0], lx, dTw);
+    build_fft_line(g.ny, ksHost.twopi_over_L[1], ly, dTw + 3 * g.nx);
+    build_fft_line(g.nz, ksHost.twopi_over_L[2], lz, dTw + 3 * (g.nx + g.ny));
     for (FftLine *l : {&lx, &ly, &lz})
         if (l->ns > kMaxStages) fail(TILD_ERR_UNSUPPORTED, "grid size factors into too many stages");
     dStep = dalloc<long long>(1);
     dKs = dalloc<KSpace>(1);
     dUk = dalloc<float>((size_t)std::max<size_t>(1, potentials.size()) * g.hstride);
     dPp = dalloc<ParticleParams>(1);
-    const int TXz = kspace_tile_width(g, (int)dfields.size(), (int)fgroups.size(), (int)potentials.size());
-    if (TXz == 0) fail(TILD_ERR_UNSUPPORTED, "the grid's z size is too large for the fused k-space pass with this many fields");
-    nblkZ = ((g.nxh + TXz - 1) / TXz) * g.ny;
+    planTransforms();
+    if (nblkZ == 0) fail(TILD_ERR_UNSUPPORTED, "the grid's z size is too large for the fused k-space pass with this many fields");
     nblkP = (int)((N + 255) / 256);
     dEpart = dalloc<double>((size_t)nblkZ * (ksHost.neterms + 6));
     dBpart = dalloc<double>((size_t)nblkP * kPartialCols);
@@ -1289,6 +1297,14 @@ void Box::allocDevice()
     sortW.na = nAnglesTot > 0 ? dalloc<uint8_t>(N) : nullptr;
     sortW.atype = nAnglesTot > 0 ? dalloc<uint8_t>(N * MAXANGLES) : nullptr;
     sortW.ang = nAnglesTot > 0 ? dalloc<int>(3 * N * MAXANGLES) : nullptr;
+}
+
+// The transform passes this box's fields take and the blocks of its k-space pass.
+void Box::planTransforms()
+{
+    const int nd = (int)dfields.size(), nfg = (int)fgroups.size();
+    twoStage = fft_two_stage(lx, ly, lz, nd, nfg);
+    nblkZ = kspace_blocks(geom, lz, nd, nfg, (int)potentials.size(), twoStage);
 }
 
 void Box::uploadParticles()
@@ -1446,26 +1462,20 @@ void Box::enqueueStep(bool energy, bool integrate, float *fout_dev)
     const Geom &g = geom;
     cudaStream_t st = stream;
     const int nd = (int)dfields.size(), nfg = (int)fgroups.size();
-    const int npair = (nd + 1) / 2;
     mark(-1);
     if (nd > 0) {
-        if (deterministic)
-            ck(launch_zero(dDepFix, sizeof(unsigned long long) * 2 * npair * g.M, st), "zero");
-        else
-            ck(launch_zero(dDep, sizeof(float2) * npair * g.M, st), "zero");
         ck(launch_deposit(g, ppHost, dX[0], dX[1], dStep, dFlags, dQ, dDep, dDepFix, deterministic, depTileCfg(), st), "deposit");
         mark(STAGE_DEPOSIT);
-        ck(launch_xfwd(g, lx, npair, nd, dDep, deterministic ? dDepFix : nullptr, dH, st), "fft x forward");
-        mark(STAGE_XFWD);
-        ck(launch_ypass(g, ly, nd, 0, dH, st), "fft y forward");
-        mark(STAGE_YFWD);
-        ck(launch_kspace_z(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, energy ? 1 : 0, nfg > 0 ? 1 : 0, nullptr, st), "kspace");
+        forwardXY();
+        if (twoStage) ck(launch_kspace2(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, energy ? 1 : 0, 1, st), "kspace");
+        else ck(launch_kspace_z(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, energy ? 1 : 0, nfg > 0 ? 1 : 0, nullptr, st), "kspace");
         if (energy && ksHost.neterms > 0) ck(launch_reduce_partials(dEpart, nblkZ, ksHost.neterms + 6, dRes, st), "reduce");
         mark(STAGE_KSPACE);
         if (nfg > 0) {
-            ck(launch_ypass(g, ly, 3 * nfg, 1, dHg, st), "fft y inverse");
+            ck(twoStage ? launch_ypass2(g, ly, nfg, 1, dHg, st) : launch_ypass(g, ly, 3 * nfg, 1, dHg, st), "fft y inverse");
             mark(STAGE_YINV);
-            ck(launch_xinv(g, lx, nfg, dHg, dRec, recLayout(), st), "fft x inverse");
+            ck(twoStage ? launch_xinv2(g, lx, nfg, dHg, dRec, recLayout(), st)
+                        : launch_xinv(g, lx, nfg, dHg, dRec, recLayout(), st), "fft x inverse");
             mark(STAGE_XINV);
         }
     }
@@ -1486,6 +1496,19 @@ void Box::enqueueStep(bool energy, bool integrate, float *fout_dev)
     }
 }
 
+// The x and y forward passes of the deposited densities.
+void Box::forwardXY()
+{
+    const Geom &g = geom;
+    const int nd = (int)dfields.size();
+    unsigned long long *df = deterministic ? dDepFix : nullptr;
+    ck(twoStage ? launch_xfwd2(g, lx, nd, dDep, df, dH, stream) : launch_xfwd(g, lx, (nd + 1) / 2, nd, dDep, df, dH, stream),
+       "fft x forward");
+    mark(STAGE_XFWD);
+    ck(twoStage ? launch_ypass2(g, ly, nd, 0, dH, stream) : launch_ypass(g, ly, nd, 0, dH, stream), "fft y forward");
+    mark(STAGE_YFWD);
+}
+
 // lastStepStart: deposit from the other position buffer, which after a step holds the
 // positions that step started from (GJF keeps x_{t-1} there, EM leaves x_t there).
 void Box::enqueueEnergyOnly(bool lastStepStart)
@@ -1493,17 +1516,12 @@ void Box::enqueueEnergyOnly(bool lastStepStart)
     const Geom &g = geom;
     cudaStream_t st = stream;
     const int nd = (int)dfields.size();
-    const int npair = (nd + 1) / 2;
     if (nd > 0 && ksHost.neterms > 0) {
-        if (deterministic)
-            ck(launch_zero(dDepFix, sizeof(unsigned long long) * 2 * npair * g.M, st), "zero");
-        else
-            ck(launch_zero(dDep, sizeof(float2) * npair * g.M, st), "zero");
         float *xa = lastStepStart ? dX[1] : dX[0], *xb = lastStepStart ? dX[0] : dX[1];
         ck(launch_deposit(g, ppHost, xa, xb, dStep, dFlags, dQ, dDep, dDepFix, deterministic, depTileCfg(), st), "deposit");
-        ck(launch_xfwd(g, lx, npair, nd, dDep, deterministic ? dDepFix : nullptr, dH, st), "fft x forward");
-        ck(launch_ypass(g, ly, nd, 0, dH, st), "fft y forward");
-        ck(launch_kspace_z(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, 1, 0, nullptr, st), "kspace energy");
+        forwardXY();
+        if (twoStage) ck(launch_kspace2(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, 1, 0, st), "kspace energy");
+        else ck(launch_kspace_z(g, lz, ksHost, dKs, dH, dUk, dHg, dEpart, 1, 0, nullptr, st), "kspace energy");
         ck(launch_reduce_partials(dEpart, nblkZ, ksHost.neterms + 6, dRes, st), "reduce");
     }
     ck(launch_bond_energy(g, ppHost, dPp, dX[0], dX[1], dStep, dBrow, dPartner, dBtype, AngleArrays{dNa, dAtype, dAng},
@@ -2479,6 +2497,7 @@ void Box::modifyBox(const std::string &rest)
                 buildPlan();
                 if ((int)dfields.size() > std::max(1, ndOld) || (int)fgroups.size() > std::max(1, nfOld))
                     fail(TILD_ERR_STATE, "plan grew after removing a potential");
+                planTransforms();
                 recMapOk = false;   // the record descriptor follows the force-group count
                 uploadFlags();
                 ck(cudaDeviceSynchronize(), "modify");

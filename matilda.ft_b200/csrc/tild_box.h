@@ -150,6 +150,8 @@ private:
     // device plan
     void buildPlan();
     void allocDevice();
+    void planTransforms();
+    void forwardXY();
     void freeDevice();
     void uploadParticles();
     void enqueueStep(bool energy, bool integrate, float *fout_dev);
@@ -230,6 +232,7 @@ private:
     ParticleParams ppHost{};
     FftLine lx{}, ly{}, lz{};
     int nblkZ = 0, nblkP = 0;
+    bool twoStage = false;          // transforms in two register stages (tild_fft2.cuh)
 
     // device state
     cudaStream_t stream = nullptr;

@@ -64,6 +64,11 @@ struct FftLine {          // Stockham mixed-radix plan of one line length
     FastDiv dP[kMaxStages];   // division by P[s]
     FastDiv dNB[kMaxStages];  // division by n / R[s]
     const float2 *tw;     // device twiddles W_n^t, t in [0, n)  (forward sign)
+    // two register stages (tild_fft2.cuh): n = r1 r2 with r2 <= r1 <= 16, or r1 = 0
+    int r1, r2;
+    FastDiv dr1, dr2;         // division by r1, r2
+    const float2 *tw2;        // W_n^{i q} at q r2 + i (i < r2, q < r1)
+    const float *kv;          // wave numbers 2 pi/L x signed index, 0 at an even n's Nyquist index
 };
 
 struct Geom {
@@ -75,6 +80,7 @@ struct Geom {
     float inv[3];              // 1.f / dxf (IEEE FP32 division)
     float L[3];
     float Lh[3];
+    FastDiv dhp, dny, dnxh;    // division by hp, ny, nxh
 };
 
 struct PotDev {
@@ -211,6 +217,7 @@ struct BatchRep {
     const KSpace *ks;
     const float *uk;
     int N, quirk4, nd, nfg, int_tile_max, dep_cap, Lx, Lxi, txz, ks_npots;
+    int two, cby, cbyi, cbz;    // two-stage transforms and their columns per block (log2)
     unsigned dq;
     float *X0, *X1, *noise;
     const uint32_t *flags;
@@ -238,8 +245,6 @@ struct BatchLaunch {        // one stage's launch over all replicas
 
 cudaError_t launch_batch_tick(const BatchRep *reps, int R, cudaStream_t st);
 // per-file pieces of the above (tild_grid.cu, tild_fft.cu, tild_particles.cu)
-void zero_batch_shape(const BatchRep &r, int deterministic, int *blocks);
-cudaError_t launch_zero_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int deterministic, cudaStream_t st);
 void deposit_batch_shape(const BatchRep &r, int deterministic, int *blocks, int *threads, size_t *smem, int *cap);
 cudaError_t launch_deposit_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int order, int nd,
                                  int deterministic, cudaStream_t st);
@@ -254,16 +259,18 @@ cudaError_t launch_particles_batch(int stage, const BatchRep *reps, int R, const
 // -------------------------------------------------------------------------------------
 // Launchers (tild_grid.cu, tild_fft.cu, tild_particles.cu, tild_sort.cu).  All run on `st`;
 // none synchronises.
-void build_fft_line(int n, FftLine &pl, float2 *dev_tw_dst);
+// plan of one axis: tables in dev[3n] (uploaded on st, complete on return)
+void build_fft_line(int n, double twopi_over_L, FftLine &pl, float2 *dev);
 void init_fft_attributes();      // opt the FFT kernels into large dynamic shared memory
 void init_deposit_attributes();  // same for the staged deposit
-cudaError_t launch_zero(void *p, size_t bytes, cudaStream_t st);
 cudaError_t launch_deposit(const Geom &g, const ParticleParams &pp, const float *X0,
                            const float *X1, const long long *d_step, const uint32_t *pflags,
                            const float *q, float2 *dep, unsigned long long *dep_fixed,
                            int deterministic, const TileCfg &tc, cudaStream_t st);
-cudaError_t launch_xfwd(const Geom &g, const FftLine &lx, int npair, int nd, const float2 *dep,
-                        const unsigned long long *dep_fixed, float2 *H, cudaStream_t st);
+// x forward pass of the packed density pairs; clears the deposit target it has read, which
+// so is all zeros between steps
+cudaError_t launch_xfwd(const Geom &g, const FftLine &lx, int npair, int nd, float2 *dep,
+                        unsigned long long *dep_fixed, float2 *H, cudaStream_t st);
 cudaError_t launch_ypass(const Geom &g, const FftLine &ly, int nfields, int inverse, float2 *H,
                          cudaStream_t st);
 cudaError_t launch_kspace_z(const Geom &g, const FftLine &lz, const KSpace &ks, const KSpace *ks_dev,
@@ -272,14 +279,46 @@ cudaError_t launch_kspace_z(const Geom &g, const FftLine &lz, const KSpace &ks, 
 // half-spectrum columns per block of the k-space z pass (4, or 2 so that its shared
 // memory fits), 0 if even 2 do not fit
 int kspace_tile_width(const Geom &g, int nd, int nfg, int npots);
+// ---- two-stage transforms (tild_fft2.cu, tild_kspace2.cu) ----
+// Whether a box's transforms run in two register stages: every axis has r1, and the box has
+// 1 to 4 density fields and as many force groups.  The inverse passes then carry two fields
+// per force group from the z pass (phi, -i k_z phi); the y pass makes the third.
+inline bool fft_two_stage(const FftLine &lx, const FftLine &ly, const FftLine &lz, int nd, int nfg)
+{
+    return lx.r1 > 0 && ly.r1 > 0 && lz.r1 > 0 && nd == nfg && nd >= 1 && nd <= 4;
+}
+cudaError_t launch_xfwd2(const Geom &g, const FftLine &lx, int nd, float2 *dep, unsigned long long *dep_fixed, float2 *H,
+                         cudaStream_t st);
+// n density fields forward, n force groups inverse
+cudaError_t launch_ypass2(const Geom &g, const FftLine &ly, int n, int inverse, float2 *H, cudaStream_t st);
+cudaError_t launch_kspace2(const Geom &g, const FftLine &lz, const KSpace &ks, const KSpace *ks_dev, const float2 *H,
+                           const float *uk, float2 *Hg, double *epart, int energy, int forces, cudaStream_t st);
+cudaError_t launch_xinv2(const Geom &g, const FftLine &lx, int nfg, const float2 *Hg, float4 *rec, const RecLayout &rl,
+                         cudaStream_t st);
+int fft2_xfwd_lines(const Geom &g, const FftLine &lx, int npair);   // lines or columns (log2) per block
+int fft2_xinv_lines(const Geom &g, const FftLine &lx, int nfg);
+int fft2_col_bits(const FftLine &l, long long ncols, int jobs);
+int kspace2_col_bits(const Geom &g, const FftLine &lz, int nf);
+// a stage's grid (bx, by), threads and shared memory with L lines or columns per block; n:
+// density fields (forward) or force groups (inverse)
+void fft2_shape(int stage, const Geom &g, const FftLine &l, int n, int L, int *bx, int *by, int *threads, size_t *smem);
+void kspace2_shape(const Geom &g, const FftLine &lz, int nf, int cb, int *blocks, int *threads, size_t *smem);
+cudaError_t launch_fft2_batch(int stage, const BatchRep *reps, int R, const BatchLaunch &bl, int deterministic,
+                              cudaStream_t st);
+cudaError_t launch_kspace2_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int nf, cudaStream_t st);
+void init_fft2_attributes();
+void init_kspace2_attributes();
+// blocks of the k-space pass over one box (the rows of its energy partials)
+int kspace_blocks(const Geom &g, const FftLine &lz, int nd, int nfg, int npots, bool two);
 // FP32 table of every potential's û(k) shape (amplitude 1) over the half spectrum
 cudaError_t launch_uk_table(const Geom &g, const KSpace *ks_dev, float *tab, cudaStream_t st);
 // S(|k|) of one real field given as float2 pairs (field in .x): x/y forward passes into
 // Hs, then the z pass bins |FFT(rho)/M|^2 into bins[3*nbins] (S, |k|, count; FP64)
 // out[m] = (rho[m], 0)
 cudaError_t launch_to_pairs(const float *rho, float2 *out, long long M, cudaStream_t st);
+// (rho_pair is cleared)
 cudaError_t launch_structure_factor(const Geom &g, const FftLine &lx, const FftLine &ly, const FftLine &lz,
-                                   const double *twopi_over_L, const float2 *rho_pair, float2 *Hs, int nbins,
+                                   const double *twopi_over_L, float2 *rho_pair, float2 *Hs, int nbins,
                                    double dk, double *bins, cudaStream_t st);
 // x inverse pass: the records of every force group, planar into rec, or into the paired
 // planes of rl when rl.paired

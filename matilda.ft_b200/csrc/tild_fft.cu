@@ -1,6 +1,7 @@
 // tild_fft.cu -- hand-written mixed-radix Stockham 3-D FFT passes fused with the
 // k-space potential/gradient multiply (sm_100a).
-#include "tild_stencil.cuh"
+#include "tild_dft.cuh"
+#include "tild_uk.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -16,129 +17,6 @@ namespace tild {
 // earlier radices: butterfly i reads i + q*n/R, twiddles by W_{pR}^{q*(i mod p)}, writes
 // (i - i mod p)*R + i mod p + q*p.  Returns the buffer holding the result.
 // =====================================================================================
-// complex arithmetic on paired FP32 instructions (FMUL2/FFMA2/FADD2 of sm_100)
-__device__ __forceinline__ float2 cmul(float2 a, float2 b)
-{
-    return __ffma2_rn(make_float2(a.y, a.y), make_float2(-b.y, b.x), __fmul2_rn(make_float2(a.x, a.x), b));
-}
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
-
-template <bool INV>
-__device__ __forceinline__ float2 twid(const float2 *tw, int t)
-{
-    float2 w = tw[t];
-    if (INV) w.y = -w.y;
-    return w;
-}
-
-__device__ __forceinline__ FastDiv make_fastdiv_dev(unsigned d)
-{
-    FastDiv f;
-    f.d = d;
-    f.m = d <= 1 ? 0u : (unsigned)((0x100000000ull + d - 1) / d);
-    return f;
-}
-
-__device__ __forceinline__ unsigned fdiv(unsigned i, const FastDiv &f)
-{
-    return f.d == 1 ? i : __umulhi(i, f.m);
-}
-
-__device__ __forceinline__ float2 mul_mi(float2 v) { return make_float2(v.y, -v.x); }   // -i v
-__device__ __forceinline__ float2 mul_pi(float2 v) { return make_float2(-v.y, v.x); }   // +i v
-
-// In-register DFT of R points, v[q] <- sum_s v[s] W_R^{+-qs} (forward sign -), R = 2, 3, 4, 5, 7, 8.
-template <bool INV>
-__device__ __forceinline__ void dft4(float2 &a0, float2 &a1, float2 &a2, float2 &a3)
-{
-    const float2 t0 = cadd(a0, a2), t1 = csub(a0, a2), t2 = cadd(a1, a3), t3 = csub(a1, a3);
-    const float2 m = INV ? mul_pi(t3) : mul_mi(t3);
-    a0 = cadd(t0, t2);
-    a1 = cadd(t1, m);
-    a2 = csub(t0, t2);
-    a3 = csub(t1, m);
-}
-
-template <bool INV, int R>
-__device__ __forceinline__ void dft_reg(float2 *v)
-{
-    if (R == 2) {
-        const float2 a = v[0], b = v[1];
-        v[0] = cadd(a, b);
-        v[1] = csub(a, b);
-    } else if (R == 4) {
-        dft4<INV>(v[0], v[1], v[2], v[3]);
-    } else if (R == 8) {
-        // radix-2 split into even and odd outputs, W_8 twiddles, two 4-point DFTs
-        const float c = 0.70710678118654752f;
-        float2 a0 = cadd(v[0], v[4]), b0 = csub(v[0], v[4]);
-        float2 a1 = cadd(v[1], v[5]), b1 = csub(v[1], v[5]);
-        float2 a2 = cadd(v[2], v[6]), b2 = csub(v[2], v[6]);
-        float2 a3 = cadd(v[3], v[7]), b3 = csub(v[3], v[7]);
-        if (INV) {
-            b1 = make_float2(c * (b1.x - b1.y), c * (b1.x + b1.y));     // * W_8^-1
-            b2 = mul_pi(b2);                                            // * W_8^-2
-            b3 = make_float2(-c * (b3.x + b3.y), c * (b3.x - b3.y));    // * W_8^-3
-        } else {
-            b1 = make_float2(c * (b1.x + b1.y), c * (b1.y - b1.x));     // * W_8^1
-            b2 = mul_mi(b2);                                            // * W_8^2
-            b3 = make_float2(c * (b3.y - b3.x), -c * (b3.x + b3.y));    // * W_8^3
-        }
-        dft4<INV>(a0, a1, a2, a3);
-        dft4<INV>(b0, b1, b2, b3);
-        v[0] = a0; v[2] = a1; v[4] = a2; v[6] = a3;
-        v[1] = b0; v[3] = b1; v[5] = b2; v[7] = b3;
-    } else if (R == 3) {
-        const float s3 = INV ? 0.86602540378443865f : -0.86602540378443865f;
-        const float2 a0 = v[0], t = cadd(v[1], v[2]), u = csub(v[1], v[2]);
-        const float2 m = make_float2(a0.x - 0.5f * t.x, a0.y - 0.5f * t.y);
-        const float2 iu = make_float2(-s3 * u.y, s3 * u.x);   // i * s3 * u
-        v[0] = cadd(a0, t);
-        v[1] = cadd(m, iu);
-        v[2] = csub(m, iu);
-    } else if (R == 5) {
-        const float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f;
-        const float s1 = INV ? -0.95105651629515357f : 0.95105651629515357f;
-        const float s2 = INV ? -0.58778525229247313f : 0.58778525229247313f;
-        const float2 a0 = v[0];
-        const float2 t1 = cadd(v[1], v[4]), t2 = cadd(v[2], v[3]), t3 = csub(v[1], v[4]), t4 = csub(v[2], v[3]);
-        const float2 m1 = make_float2(a0.x + c1 * t1.x + c2 * t2.x, a0.y + c1 * t1.y + c2 * t2.y);
-        const float2 m2 = make_float2(a0.x + c2 * t1.x + c1 * t2.x, a0.y + c2 * t1.y + c1 * t2.y);
-        // n1 = s1 t3 + s2 t4, n2 = s2 t3 - s1 t4; b1 = m1 - i n1, b4 = m1 + i n1,
-        // b2 = m2 - i n2, b3 = m2 + i n2
-        const float2 n1 = make_float2(s1 * t3.x + s2 * t4.x, s1 * t3.y + s2 * t4.y);
-        const float2 n2 = make_float2(s2 * t3.x - s1 * t4.x, s2 * t3.y - s1 * t4.y);
-        v[0] = make_float2(a0.x + t1.x + t2.x, a0.y + t1.y + t2.y);
-        v[1] = make_float2(m1.x + n1.y, m1.y - n1.x);
-        v[4] = make_float2(m1.x - n1.y, m1.y + n1.x);
-        v[2] = make_float2(m2.x + n2.y, m2.y - n2.x);
-        v[3] = make_float2(m2.x - n2.y, m2.y + n2.x);
-    } else if (R == 7) {
-        // t_k = a_k + a_{7-k}, u_k = a_k - a_{7-k}; b_q = m_q -+ i n_q with
-        // m_q = a0 + sum_k cos(2 pi qk/7) t_k, n_q = sum_k sin(2 pi qk/7) u_k
-        const float c1 = 0.62348980185873359f, c2 = -0.22252093395631434f, c3 = -0.90096886790241903f;
-        const float sg = INV ? -1.f : 1.f;
-        const float s1 = sg * 0.78183148246802980f, s2 = sg * 0.97492791218182362f, s3 = sg * 0.43388373911755823f;
-        const float2 a0 = v[0];
-        const float2 t1 = cadd(v[1], v[6]), t2 = cadd(v[2], v[5]), t3 = cadd(v[3], v[4]);
-        const float2 u1 = csub(v[1], v[6]), u2 = csub(v[2], v[5]), u3 = csub(v[3], v[4]);
-        const float2 m1 = make_float2(a0.x + c1 * t1.x + c2 * t2.x + c3 * t3.x, a0.y + c1 * t1.y + c2 * t2.y + c3 * t3.y);
-        const float2 m2 = make_float2(a0.x + c2 * t1.x + c3 * t2.x + c1 * t3.x, a0.y + c2 * t1.y + c3 * t2.y + c1 * t3.y);
-        const float2 m3 = make_float2(a0.x + c3 * t1.x + c1 * t2.x + c2 * t3.x, a0.y + c3 * t1.y + c1 * t2.y + c2 * t3.y);
-        const float2 n1 = make_float2(s1 * u1.x + s2 * u2.x + s3 * u3.x, s1 * u1.y + s2 * u2.y + s3 * u3.y);
-        const float2 n2 = make_float2(s2 * u1.x - s3 * u2.x - s1 * u3.x, s2 * u1.y - s3 * u2.y - s1 * u3.y);
-        const float2 n3 = make_float2(s3 * u1.x - s1 * u2.x + s2 * u3.x, s3 * u1.y - s1 * u2.y + s2 * u3.y);
-        v[0] = make_float2(a0.x + t1.x + t2.x + t3.x, a0.y + t1.y + t2.y + t3.y);
-        v[1] = cadd(m1, mul_mi(n1));
-        v[6] = csub(m1, mul_mi(n1));
-        v[2] = cadd(m2, mul_mi(n2));
-        v[5] = csub(m2, mul_mi(n2));
-        v[3] = cadd(m3, mul_mi(n3));
-        v[4] = csub(m3, mul_mi(n3));
-    }
-}
-
 // One radix-R Stockham stage over L lines: butterfly i of line l reads i + q*nb, is
 // twiddled by W_{pR}^{q*(i mod p)} and writes (i - i mod p)*R + i mod p + q*p.
 template <bool INV, int R>
@@ -168,7 +46,7 @@ __device__ __forceinline__ void fft_stage(const float2 *__restrict__ src, float2
 #pragma unroll
             for (int q = 1; q < R; q++) v[q] = cmul(v[q], twid<INV>(tw, q * ks));
         }
-        dft_reg<INV, R>(v);
+        dft<INV, R>(v);
 #pragma unroll
         for (int q = 0; q < R; q++) dst[db + q * sp] = v[q];
     }
@@ -301,8 +179,8 @@ __device__ __forceinline__ void tile_load_async(float2 *dst, int dpitch, const f
 // FFT A(k) = (Z(k) + conj Z(n-k))/2 and B(k) = (Z(k) - conj Z(n-k))/(2i), k in [0, n/2].
 // -------------------------------------------------------------------------------------
 template <bool FIXED>
-__device__ __forceinline__ void xfwd_body(const Geom &g, const FftLine &lx, int nd, const float2 *__restrict__ dep,
-                                          const unsigned long long *__restrict__ depfix, double fscale,
+__device__ __forceinline__ void xfwd_body(const Geom &g, const FftLine &lx, int nd, float2 *__restrict__ dep,
+                                          unsigned long long *__restrict__ depfix, double fscale,
                                           float2 *__restrict__ H, int L, unsigned vbx, unsigned vby)
 {
     extern __shared__ __align__(16) float2 sm[];
@@ -336,6 +214,16 @@ __device__ __forceinline__ void xfwd_body(const Geom &g, const FftLine &lx, int 
         }
     }
     __syncthreads();
+    // the rows are this block's alone: clear them for the next step's deposit
+    for (int e = threadIdx.x; e < lv * n; e += blockDim.x) {
+        const long long idx = line0 * n + e;
+        if (FIXED) {
+            depfix[(2 * pair) * g.M + idx] = 0ull;
+            if (2 * pair + 1 < nd) depfix[(2 * pair + 1) * g.M + idx] = 0ull;
+        } else {
+            dep[pair * g.M + idx] = make_float2(0.f, 0.f);
+        }
+    }
     const float2 *R = fft_lines<false>(A, B, L, n, 1, lx, tw, false, make_fastdiv_dev(L));
     const int nxh = g.nxh;
     const FastDiv dh = make_fastdiv_dev((unsigned)nxh);
@@ -351,8 +239,8 @@ __device__ __forceinline__ void xfwd_body(const Geom &g, const FftLine &lx, int 
     }
 }
 template <bool FIXED>
-__global__ void __launch_bounds__(256) k_xfwd(Geom g, FftLine lx, int nd, const float2 *__restrict__ dep,
-                                              const unsigned long long *__restrict__ depfix,
+__global__ void __launch_bounds__(256) k_xfwd(Geom g, FftLine lx, int nd, float2 *__restrict__ dep,
+                                              unsigned long long *__restrict__ depfix,
                                               double fscale, float2 *__restrict__ H, int L)
 {
     xfwd_body<FIXED>(g, lx, nd, dep, depfix, fscale, H, L, blockIdx.x, blockIdx.y);
@@ -409,53 +297,6 @@ __global__ void __launch_bounds__(256, 6) k_ypass_batch(const BatchRep *__restri
     const unsigned lb = blockIdx.x - pre[r];
     const unsigned gx = (unsigned)((b.g.nxh + TX - 1) / TX), gy = (unsigned)b.g.nz;
     ypass_body<INV, TX>(b.g, b.ly, INV ? b.Hg : b.H, lb % gx, (lb / gx) % gy, lb / (gx * gy));
-}
-
-// û(k) of each potential kind, FP64 (ps_potentialGaussian.cu:38-46,
-// ps_potentialErf2.cu:111-124, ps_potentialErfG.cu:177-190, ps_potentialCharges.cu:241-258),
-// as amplitude x shape: the shape is fixed for a box, the amplitude follows the ramp.
-__device__ double uk_shape(const PotDev &p, double k2)
-{
-    const double PI4 = 12.566370614359172953850573533118;
-    if (p.kind == POT_WALL) return 0.0;   // a per-particle term, nothing in k-space
-    if (p.kind == POT_GAUSSIAN) return exp(-0.5 * k2 * p.sig2);
-    if (p.kind == POT_CHARGES) return k2 > 0.0 ? PI4 * p.lB * exp(-k2 * p.sig2) / k2 : 0.0;
-    const double R = p.Rp;
-    double t;
-    if (k2 == 0.0) {
-        t = PI4 * R * R * R / 3.0;
-        return p.kind == POT_ERF2 ? t * t : t;
-    }
-    const double k = sqrt(k2);
-    double sn, cs;
-    sincos(R * k, &sn, &cs);
-    t = PI4 * (sn - R * k * cs) / (k2 * k);
-    const double gs = exp(-0.5 * k2 * p.sig2);
-    return p.kind == POT_ERF2 ? gs * t * t : gs * t;
-}
-
-__device__ __forceinline__ double uk_amp(const PotDev &p) { return p.kind == POT_CHARGES ? 1.0 : p.amp; }
-
-__device__ __forceinline__ double uk_eval(const PotDev &p, double k2) { return uk_amp(p) * uk_shape(p, k2); }
-
-// (d û / d k) / k for k > 0, FP64, amplitude included: the strain derivative of the pair
-// energy.  gaussian: -sigma^2 û; charges: û (-2 sigma^2 - 2/k^2); erf2/erfG with
-// t = 4 pi (sin Rk - Rk cos Rk)/k^3: A g t^(p-1) (-sigma^2 t + p t'/k),
-// t'/k = 4 pi (R^2 sin(Rk)/k^3 - 3 (sin Rk - Rk cos Rk)/k^5).
-__device__ double uk_dk_over_k(const PotDev &p, double k2)
-{
-    if (k2 <= 0.0 || p.kind == POT_WALL) return 0.0;
-    if (p.kind == POT_GAUSSIAN) return -p.sig2 * uk_eval(p, k2);
-    if (p.kind == POT_CHARGES) return uk_eval(p, k2) * (-2.0 * p.sig2 - 2.0 / k2);
-    const double PI4 = 12.566370614359172953850573533118;
-    const double R = p.Rp, k = sqrt(k2);
-    double sn, cs;
-    sincos(R * k, &sn, &cs);
-    const double f = sn - R * k * cs;
-    const double t = PI4 * f / (k2 * k);
-    const double dt_k = PI4 * (R * R * sn / (k2 * k) - 3.0 * f / (k2 * k2 * k));
-    const double gs = exp(-0.5 * k2 * p.sig2);
-    return p.kind == POT_ERF2 ? p.amp * gs * t * (-p.sig2 * t + 2.0 * dt_k) : p.amp * gs * (-p.sig2 * t + dt_k);
 }
 
 __device__ __forceinline__ int signed_index(int i, int n) { return (i < n - i) ? i : i - n; }
@@ -828,9 +669,11 @@ void init_fft_attributes()
     set_max_smem(k_kspace_batch<4>, kKspaceSmemMax);
     set_max_smem(k_kspace_batch<2>, kKspaceSmemMax);
     set_max_smem(k_xinv_batch, 200 * 1024);
+    init_fft2_attributes();
+    init_kspace2_attributes();
 }
 
-void build_fft_line(int n, FftLine &pl, float2 *dev_tw_dst)
+void build_fft_line(int n, double twopi_over_L, FftLine &pl, float2 *dev)
 {
     pl.n = n;
     pl.ns = 0;
@@ -863,12 +706,29 @@ void build_fft_line(int n, FftLine &pl, float2 *dev_tw_dst)
         const double a = -2.0 * M_PI * (double)t / (double)n;
         tw[t] = make_float2((float)cos(a), (float)sin(a));
     }
-    cudaMemcpy(dev_tw_dst, tw.data(), n * sizeof(float2), cudaMemcpyHostToDevice);
-    pl.tw = dev_tw_dst;
+    // two register stages: the most balanced factors r2 <= r1 <= 16, if there are any
+    pl.r1 = pl.r2 = 0;
+    for (int r = 1; r <= 16 && !pl.r1; r++)
+        if (r * r >= n && n % r == 0) {
+            pl.r1 = r;
+            pl.r2 = n / r;
+        }
+    pl.dr1 = make_fastdiv((unsigned)std::max(1, pl.r1));
+    pl.dr2 = make_fastdiv((unsigned)std::max(1, pl.r2));
+    std::vector<float2> all(3 * (size_t)n, make_float2(0.f, 0.f));
+    std::copy(tw.begin(), tw.end(), all.begin());
+    for (int q = 0; q < pl.r1; q++)
+        for (int i = 0; i < pl.r2; i++) all[n + q * pl.r2 + i] = tw[q * i];
+    float *kv = reinterpret_cast<float *>(all.data() + 2 * n);
+    for (int i = 0; i < n; i++) kv[i] = 2 * i == n ? 0.f : (float)(twopi_over_L * (i < n - i ? i : i - n));
+    cudaMemcpy(dev, all.data(), all.size() * sizeof(float2), cudaMemcpyHostToDevice);
+    pl.tw = dev;
+    pl.tw2 = dev + n;
+    pl.kv = reinterpret_cast<const float *>(dev + 2 * n);
 }
 
-cudaError_t launch_xfwd(const Geom &g, const FftLine &lx, int npair, int nd, const float2 *dep,
-                        const unsigned long long *dep_fixed, float2 *H, cudaStream_t st)
+cudaError_t launch_xfwd(const Geom &g, const FftLine &lx, int npair, int nd, float2 *dep,
+                        unsigned long long *dep_fixed, float2 *H, cudaStream_t st)
 {
     const int L = lines_per_block(g.nx);
     const long long nlines = (long long)g.ny * g.nz;
@@ -954,6 +814,18 @@ cudaError_t launch_xinv(const Geom &g, const FftLine &lx, int nfg, const float2 
     return cudaGetLastError();
 }
 
+int kspace_blocks(const Geom &g, const FftLine &lz, int nd, int nfg, int npots, bool two)
+{
+    if (!two) {
+        const int tx = kspace_tile_width(g, nd, nfg, npots);
+        return tx ? ((g.nxh + tx - 1) / tx) * g.ny : 0;
+    }
+    int nb, thr;
+    size_t sm;
+    kspace2_shape(g, lz, nd, kspace2_col_bits(g, lz, nd), &nb, &thr, &sm);
+    return nb;
+}
+
 // ---- batched replicas: shapes and launches of the transform stages ----
 int fft_batch_lines(int stage, const Geom &g, int nfg)
 {
@@ -963,6 +835,18 @@ int fft_batch_lines(int stage, const Geom &g, int nfg)
 void fft_batch_shape(int stage, const BatchRep &r, int *blocks, int *threads, size_t *smem)
 {
     const Geom &g = r.g;
+    if (r.two) {
+        int bx, by = 1;
+        switch (stage) {
+            case BS_XFWD: fft2_shape(stage, g, r.lx, r.nd, r.Lx, &bx, &by, threads, smem); break;
+            case BS_YFWD: fft2_shape(stage, g, r.ly, r.nd, 1 << r.cby, &bx, &by, threads, smem); break;
+            case BS_YINV: fft2_shape(stage, g, r.ly, r.nfg, 1 << r.cbyi, &bx, &by, threads, smem); break;
+            case BS_KSPACE: kspace2_shape(g, r.lz, r.nd, r.cbz, &bx, threads, smem); break;
+            default: fft2_shape(stage, g, r.lx, r.nfg, r.Lxi, &bx, &by, threads, smem); break;
+        }
+        *blocks = bx * by;
+        return;
+    }
     const long long nlines = (long long)g.ny * g.nz;
     *threads = 256;
     switch (stage) {
@@ -1014,11 +898,11 @@ cudaError_t launch_uk_table(const Geom &g, const KSpace *ks_dev, float *tab, cud
 }
 
 cudaError_t launch_structure_factor(const Geom &g, const FftLine &lx, const FftLine &ly, const FftLine &lz,
-                                   const double *twopi_over_L, const float2 *rho_pair, float2 *Hs, int nbins,
+                                   const double *twopi_over_L, float2 *rho_pair, float2 *Hs, int nbins,
                                    double dk, double *bins, cudaStream_t st)
 {
-    cudaError_t e = launch_xfwd(g, lx, 1, 1, rho_pair, nullptr, Hs, st);
-    if (e == cudaSuccess) e = launch_ypass(g, ly, 1, 0, Hs, st);
+    cudaError_t e = lx.r1 ? launch_xfwd2(g, lx, 1, rho_pair, nullptr, Hs, st) : launch_xfwd(g, lx, 1, 1, rho_pair, nullptr, Hs, st);
+    if (e == cudaSuccess) e = ly.r1 ? launch_ypass2(g, ly, 1, 0, Hs, st) : launch_ypass(g, ly, 1, 0, Hs, st);
     if (e != cudaSuccess) return e;
     constexpr int TX = kTXz;
     dim3 grid((g.nxh + TX - 1) / TX, g.ny);

@@ -98,9 +98,6 @@ __global__ void k_group_density_frames(Geom g, int quirk4, const float *X0, cons
             }
 }
 
-// ---- launchers ----
-cudaError_t launch_zero(void *p, size_t bytes, cudaStream_t st) { return cudaMemsetAsync(p, 0, bytes, st); }
-
 // -------------------------------------------------------------------------------------
 // Shared-memory staged deposit for spatially sorted particles.  Each CTA takes
 // kDepPB consecutive slots, finds the box of grid points their stencils cover (relative
@@ -447,34 +444,6 @@ static void dep_launch(const Geom &g, const ParticleParams &pp, const float *X0,
         dep_launch_nf<P, 2>(nb, threads, g, pp, X0, X1, d_step, pflags, q, dep, depfix, tc, st);
     else
         dep_launch_nf<P, 0>(nb, threads, g, pp, X0, X1, d_step, pflags, q, dep, depfix, tc, st);
-}
-
-// zero every replica's deposit target: 8-byte words (float2 pairs, or 64-bit fixed point
-// in deterministic mode), 2048 per CTA
-__global__ void k_zero_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre, int R, int fixed)
-{
-    const int r = batch_replica(pre, R, blockIdx.x);
-    const BatchRep &b = reps[r];
-    const long long words = (long long)(fixed ? 2 : 1) * ((b.nd + 1) / 2) * b.g.M;
-    unsigned long long *p = fixed ? b.depfix : reinterpret_cast<unsigned long long *>(b.dep);
-    const long long i0 = (long long)(blockIdx.x - pre[r]) * 2048 + threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < 8; k++) {
-        const long long i = i0 + k * 256;
-        if (i < words) p[i] = 0ull;
-    }
-}
-
-void zero_batch_shape(const BatchRep &r, int deterministic, int *blocks)
-{
-    const long long words = (long long)(deterministic ? 2 : 1) * ((r.nd + 1) / 2) * r.g.M;
-    *blocks = (int)((words + 2047) / 2048);
-}
-
-cudaError_t launch_zero_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int deterministic, cudaStream_t st)
-{
-    k_zero_batch<<<bl.blocks, 256, 0, st>>>(reps, bl.pre, R, deterministic);
-    return cudaGetLastError();
 }
 
 void deposit_batch_shape(const BatchRep &r, int deterministic, int *blocks, int *threads, size_t *smem, int *cap)
