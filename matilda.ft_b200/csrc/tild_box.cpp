@@ -1140,6 +1140,7 @@ void Box::buildPlan()
     ks.nfg = (int)fgroups.size();
     ks.nd = (int)dfields.size();
     for (int j = 0; j < 3; j++) ks.twopi_over_L[j] = 2.0 * M_PI / (double)L[j];
+    kspace2_coefficients(ks);
 
     // particle params
     ParticleParams &pp = ppHost;
@@ -1597,6 +1598,7 @@ void Box::updateRamps(int64_t step, int64_t maxSteps)
         ksHost.pots[pi].amp = p.amp_eff;
     }
     if (!any) return;
+    kspace2_coefficients(ksHost);
     *hKsPinned = ksHost;
     ck(cudaMemcpyAsync(dKs, hKsPinned, sizeof(KSpace), cudaMemcpyHostToDevice, stream), "ramp upload");
     ck(cudaStreamSynchronize(stream), "ramp sync");

@@ -114,6 +114,8 @@ struct KSpace {
     int neterms;
     ETerm eterms[kMaxPots];
     double twopi_over_L[3];
+    // coefficients of the two-stage pass: phi_f += cm[(p nd + f) nd + d] u_p(k) rhohat_d (nd = nfg <= 4)
+    float cm[kMaxPots * 16];
 };
 
 struct TypeCoef {   // per-type integrator constants (ps_integratorGJF.cu:63-76)
@@ -308,6 +310,8 @@ cudaError_t launch_fft2_batch(int stage, const BatchRep *reps, int R, const Batc
 cudaError_t launch_kspace2_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int nf, cudaStream_t st);
 void init_fft2_attributes();
 void init_kspace2_attributes();
+// fills ks.cm from its terms and the potentials' amplitudes
+void kspace2_coefficients(KSpace &ks);
 // blocks of the k-space pass over one box (the rows of its energy partials)
 int kspace_blocks(const Geom &g, const FftLine &lz, int nd, int nfg, int npots, bool two);
 // FP32 table of every potential's û(k) shape (amplitude 1) over the half spectrum

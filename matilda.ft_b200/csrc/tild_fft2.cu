@@ -136,34 +136,29 @@ __global__ void __launch_bounds__(256, 3) k_xfwd2_batch(const BatchRep *__restri
 // blocks tile nz hp columns without a remainder per plane.
 // -------------------------------------------------------------------------------------
 template <bool INV, int R1, bool GRAD>
-__device__ __forceinline__ void y_stage1(const FftLine &ly, const float2 *__restrict__ src, float2 *S, int set, int hp,
-                                         int cb, int c, int i, bool grad)
+__device__ __forceinline__ void y_stage1(const FftLine &ly, float2 *d, int set, int cb, int i, bool grad)
 {
     const int r2 = ly.r2;
     float2 v[R1];
-    col_load<R1>(v, src + i * hp, r2 * hp);
-    float2 *d = S + (i << cb) + c;
     if (GRAD && grad) {   // -i k_y times the spectrum, a transform of its own in the second set
-        float2 w[R1];
+        col_load<R1>(v, d, r2 << cb);
 #pragma unroll
-        for (int q = 0; q < R1; q++) {
-            const float k = __ldg(ly.kv + i + r2 * q);
-            w[q] = mul_mik(k, v[q]);
-        }
-        stage1_reg<INV, R1>(w, ly.tw2, r2, i);
-        col_store<R1>(w, d + set, r2 << cb);
+        for (int q = 0; q < R1; q++) v[q] = mul_mik(__ldg(ly.kv + i + r2 * q), v[q]);
+        stage1_reg<INV, R1>(v, ly.tw2, r2, i);
+        col_store<R1>(v, d + set, r2 << cb);
     }
+    col_load<R1>(v, d, r2 << cb);
     stage1_reg<INV, R1>(v, ly.tw2, r2, i);
     col_store<R1>(v, d, r2 << cb);
 }
 
 template <bool INV, int R2>
-__device__ __forceinline__ void y_stage2(const float2 *S, float2 *__restrict__ dst, int r1, int hp, int cb, int c, int k1)
+__device__ __forceinline__ void y_stage2(const float2 *S, float2 *__restrict__ dst, int r1, int hp, int cb)
 {
     float2 v[R2];
-    col_load<R2>(v, S + ((k1 * R2) << cb) + c, 1 << cb);
+    col_load<R2>(v, S, 1 << cb);
     dft<INV, R2>(v);
-    col_store<R2>(v, dst + k1 * hp, r1 * hp);
+    col_store<R2>(v, dst, r1 * hp);
 }
 
 // F: the field's half spectrum (transformed in place); grad (inverse only): the spectrum
@@ -174,31 +169,40 @@ __device__ __forceinline__ void ypass2_body(const Geom &g, const FftLine &ly, fl
 {
     extern __shared__ __align__(16) float2 sm[];
     const int r1 = ly.r1, r2 = ly.r2, tid = threadIdx.x, c = tid & ((1 << cb) - 1), i = tid >> cb;
+    const int ncol = g.nz * g.hp;
+    {   // column pairs never straddle two planes (hp is a multiple of 4); the padding columns
+        // are copied and transformed with the rest and not written back
+        const int cc = (tid & ((1 << (cb - 1)) - 1)) * 2, j = (int)(vbx << cb) + cc, z = (int)fdiv((unsigned)j, g.dhp);
+        if (j < ncol) col_stage(sm, F + (long long)z * g.ny * g.hp + (j - z * g.hp), g.hp, g.ny, cb, cc);
+    }
     const int j = (int)(vbx << cb) + c, z = (int)fdiv((unsigned)j, g.dhp), kx = j - z * g.hp;
-    const bool col = z < g.nz && kx < g.nxh;
+    const bool col = j < ncol && kx < g.nxh;
     float2 *base = F + (long long)z * g.ny * g.hp + kx;
     const int set = g.ny << cb;
+    col_stage_wait();
+    __syncthreads();
     if (col && i < r2) {
-#define TILD_Y1(R) y_stage1<INV, R, INV>(ly, base, sm, set, g.hp, cb, c, i, grad)
+#define TILD_Y1(R) y_stage1<INV, R, INV>(ly, sm + (i << cb) + c, set, cb, i, grad)
         TILD_RADIX(r1, TILD_Y1)
 #undef TILD_Y1
     }
     __syncthreads();
     if (col && i < r1) {
-#define TILD_Y2(R)                                                                                   \
-    do {                                                                                             \
-        y_stage2<INV, R>(sm, base, r1, g.hp, cb, c, i);                                              \
-        if (INV && grad) y_stage2<INV, R>(sm + set, base + g.hstride, r1, g.hp, cb, c, i);           \
-    } while (0)
-        TILD_RADIX(r2, TILD_Y2)
+#pragma unroll 1
+        for (int t = 0; t <= (INV && grad ? 1 : 0); t++) {
+            const float2 *s = sm + t * set + ((i * r2) << cb) + c;
+            float2 *d = base + t * g.hstride + i * g.hp;
+#define TILD_Y2(R) y_stage2<INV, R>(s, d, r1, g.hp, cb)
+            TILD_RADIX(r2, TILD_Y2)
 #undef TILD_Y2
+        }
     }
 }
 
 // forward: block (x, field); inverse: block (x, 2 f) takes phi_f (field 3f) into the x and y
 // gradients' fields 3f and 3f + 1, block (x, 2 f + 1) the z gradient 3f + 2
 template <bool INV>
-__global__ void __launch_bounds__(256, 3) k_ypass2(Geom g, FftLine ly, float2 *__restrict__ H, int cb)
+__global__ void __launch_bounds__(256, 4) k_ypass2(Geom g, FftLine ly, float2 *__restrict__ H, int cb)
 {
     const unsigned y = blockIdx.y;
     float2 *F = H + (long long)(INV ? 3 * (y >> 1) + 2 * (y & 1) : y) * g.hstride;
@@ -206,7 +210,7 @@ __global__ void __launch_bounds__(256, 3) k_ypass2(Geom g, FftLine ly, float2 *_
 }
 
 template <bool INV>
-__global__ void __launch_bounds__(256, 3) k_ypass2_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre, int R)
+__global__ void __launch_bounds__(256, 4) k_ypass2_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre, int R)
 {
     const int r = batch_replica(pre, R, blockIdx.x);
     const BatchRep &b = reps[r];
@@ -224,28 +228,34 @@ __global__ void __launch_bounds__(256, 3) k_ypass2_batch(const BatchRep *__restr
 // Fields 3f hold phi_f after the y pass: times -i k_x here.  A thread of the second stage
 // ends with r2 points of all three pairs, so the records go out as whole float4/float2.
 // -------------------------------------------------------------------------------------
+// First stage of a pair's lines in place: a and b are the staged rows of the two fields in the
+// line's region of the exchange, d its element (0, i); every thread of the block reaches the
+// barrier between the reads and the writes
 template <int R1>
-__device__ __forceinline__ void xi_stage1(const FftLine &lx, const float2 *__restrict__ ra, const float2 *__restrict__ rb,
-                                          bool gradx, int nxh, float2 *d, int i)
+__device__ __forceinline__ void xi_stage1(const FftLine &lx, float2 *d, int hp, int nxh, int i, bool two, bool grada,
+                                          bool act)
 {
     const int n = lx.n, r2 = lx.r2, r2p = r2 | 1;
     float2 v[R1];
+    if (act) {
+        const float2 *ra = d - i;
 #pragma unroll
-    for (int q = 0; q < R1; q++) {
-        const int k = i + r2 * q;
-        const bool direct = k < nxh;
-        const int kk = direct ? k : n - k;
-        float2 a = ra[kk], b = rb ? rb[kk] : make_float2(0.f, 0.f);
-        if (gradx) {
-            const float kx = __ldg(lx.kv + kk);
-            a = mul_mik(kx, a);
+        for (int q = 0; q < R1; q++) {
+            const int k = i + r2 * q;
+            const bool direct = k < nxh;
+            const int kk = direct ? k : n - k;
+            float2 a = ra[kk], b = two ? ra[hp + kk] : make_float2(0.f, 0.f);
+            if (grada) a = mul_mik(__ldg(lx.kv + kk), a);
+            if (kk == 0 || 2 * kk == n) a.y = b.y = 0.f;
+            v[q] = direct ? cadd(a, make_float2(-b.y, b.x)) : cadd(make_float2(a.x, -a.y), make_float2(b.y, b.x));
         }
-        if (kk == 0 || 2 * kk == n) a.y = b.y = 0.f;
-        v[q] = direct ? cadd(a, make_float2(-b.y, b.x)) : cadd(make_float2(a.x, -a.y), make_float2(b.y, b.x));
+        stage1_reg<true, R1>(v, lx.tw2, r2, i);
     }
-    stage1_reg<true, R1>(v, lx.tw2, r2, i);
+    __syncthreads();
+    if (act) {
 #pragma unroll
-    for (int q = 0; q < R1; q++) d[q * r2p] = v[q];
+        for (int q = 0; q < R1; q++) d[q * r2p] = v[q];
+    }
 }
 
 template <int R2>
@@ -256,76 +266,109 @@ __device__ __forceinline__ void xi_load(float2 *v, const float2 *s)
     dft<true, R2>(v);
 }
 
-// second stage of one line's k1 and the records: p0 = (x, y) of the first group, p1 of the
-// second, p2 = (z, z); E: the exchange of pair 0, pairs `set` apart
+// The points x = k1 + r1 k (k < R2) of a line's records, at the point and at every ghost of it:
+// the padded coordinates c' in [-gl, n + gh) with c' = c mod n along each axis.
+template <int R2, typename T, typename F>
+__device__ __forceinline__ void xi_emit(const Geom &g, const RecLayout &rl, T *__restrict__ plane, int line, int k1, int r1,
+                                        F value)
+{
+    const int gl = rl.gl, n = g.nx;
+    const int z = (int)fdiv((unsigned)line, g.dny), y = line - z * g.ny;
+    // the lowest copy: c itself, or c - m within gl of the top (an axis has order + 2 points or
+    // more, so gl = order / 2 + 1 layers hold at most one copy)
+    auto low = [gl](int c, int m) { return c + gl < m ? c : c - m; };
+    for (int zz = low(z, g.nz); zz < g.nz + rl.gh[2]; zz += g.nz)
+        for (int yy = low(y, g.ny); yy < g.ny + rl.gh[1]; yy += g.ny) {
+            T *row = plane + ((long long)(zz + gl) * rl.py + (yy + gl)) * rl.px + gl;
+#pragma unroll
+            for (int k = 0; k < R2; k++) {
+                const int x = k1 + r1 * k;
+                const T v = value(k);
+                row[x] = v;
+                if (x < rl.gh[0] || x >= n - gl)
+                    for (int xx = low(x, n); xx < n + rl.gh[0]; xx += n)
+                        if (xx != x) row[xx] = v;
+            }
+        }
+}
+
+// second stage of one line's k1 and the records: pair 0 is (x, y) of the first group, pair 1
+// of the second, pair 2 (z, z); E: the exchange of pair 0, pairs `set` apart.  Two pairs at a
+// time in registers: plane A (g0.x, g0.y, g1.x, g1.y) or (x, y, z, 0), then plane B (g0.z, g1.z).
 template <int R2>
 __device__ __forceinline__ void xi_stage2(const Geom &g, const float2 *E, int set, int r1, int k1, bool g2, int line,
                                           float4 *__restrict__ rec, const RecLayout &rl)
 {
-    float2 p0[R2], p1[R2], p2[R2];
-    xi_load<R2>(p0, E);
-    if (g2) xi_load<R2>(p1, E + set);
-    xi_load<R2>(p2, E + 2 * set);
-    if (!rl.paired) {   // planar records of the group(s)
-        float4 *r = rec + (long long)line * g.nx + k1;
-#pragma unroll
-        for (int k = 0; k < R2; k++) {
-            r[k * r1] = make_float4(p0[k].x, p0[k].y, p2[k].x, 0.f);
-            if (g2) r[g.M + k * r1] = make_float4(p1[k].x, p1[k].y, p2[k].y, 0.f);
+    float2 p[R2], s[R2];
+    xi_load<R2>(p, E);
+    if (rl.paired) {
+        xi_load<R2>(s, E + (g2 ? 1 : 2) * set);
+        xi_emit<R2>(g, rl, rl.A, line, k1, r1, [&](int k) { return make_float4(p[k].x, p[k].y, s[k].x, g2 ? s[k].y : 0.f); });
+        if (g2) {
+            xi_load<R2>(p, E + 2 * set);
+            xi_emit<R2>(g, rl, rl.B, line, k1, r1, [&](int k) { return p[k]; });
         }
         return;
     }
-    // plane A (g0.x, g0.y, g1.x, g1.y) or (x, y, z, 0), plane B (g0.z, g1.z), at the point
-    // and at every ghost of it: the padded coordinates c' in [-gl, n + gh) with c' = c mod n
-    const int gl = rl.gl, n = g.nx;
-    const int z = (int)fdiv((unsigned)line, g.dny), y = line - z * g.ny;
-    auto low = [gl](int c, int m) { return c + gl < m ? c : c - m * ((c + gl) / m); };
-    for (int zz = low(z, g.nz); zz < g.nz + rl.gh[2]; zz += g.nz)
-        for (int yy = low(y, g.ny); yy < g.ny + rl.gh[1]; yy += g.ny) {
-            const long long rb = ((long long)(zz + gl) * rl.py + (yy + gl)) * rl.px + gl;
-            float4 *A = rl.A + rb + k1;
-            float2 *B = g2 ? rl.B + rb + k1 : nullptr;
+    xi_load<R2>(s, E + 2 * set);
+    float4 *r = rec + (long long)line * g.nx + k1;   // planar records of the group(s)
 #pragma unroll
-            for (int k = 0; k < R2; k++) {
-                const float4 a = g2 ? make_float4(p0[k].x, p0[k].y, p1[k].x, p1[k].y)
-                                    : make_float4(p0[k].x, p0[k].y, p2[k].x, 0.f);
-                A[k * r1] = a;
-                if (g2) B[k * r1] = p2[k];
-                const int x = k1 + r1 * k;
-                if (x < rl.gh[0] || x >= n - gl)
-                    for (int xx = low(x, n); xx < n + rl.gh[0]; xx += n) {
-                        if (xx == x) continue;
-                        rl.A[rb + xx] = a;
-                        if (g2) rl.B[rb + xx] = p2[k];
-                    }
-            }
-        }
+    for (int k = 0; k < R2; k++) r[k * r1] = make_float4(p[k].x, p[k].y, s[k].x, 0.f);
+    if (g2) {
+        xi_load<R2>(p, E + set);
+#pragma unroll
+        for (int k = 0; k < R2; k++) r[g.M + k * r1] = make_float4(p[k].x, p[k].y, s[k].y, 0.f);
+    }
+}
+
+// a line's region of a pair's exchange: r1 rows of r2 (made odd) values, and before that the
+// two staged rows; even, so that rows are 16-byte aligned, and r2 or r2 + 1 (mod 16), so that
+// consecutive threads (l, i) fall on (nearly) consecutive values
+__host__ __device__ inline int xi_pitch(int r1, int r2, int hp)
+{
+    const int p = r1 * (r2 | 1) > 2 * hp ? r1 * (r2 | 1) : 2 * hp, even = (r2 + 1) & ~1;
+    return p + ((even - p) & 15);
 }
 
 __device__ __forceinline__ void xinv2_body(const Geom &g, const FftLine &lx, int nfg, const float2 *__restrict__ Hg,
                                            float4 *__restrict__ rec, const RecLayout &rl, int L, unsigned vbx, unsigned h)
 {
     extern __shared__ __align__(16) float2 sm[];
-    const int r1 = lx.r1, r2 = lx.r2, lp = x_pitch(r1, r2), set = L * lp, tid = threadIdx.x;
+    const int r1 = lx.r1, r2 = lx.r2, lp = xi_pitch(r1, r2, g.hp), set = L * lp, tid = threadIdx.x, hp = g.hp;
     const bool g2 = (int)(2 * h + 1) < nfg;
     const long long nlines = (long long)g.ny * g.nz, line0 = (long long)vbx * L;
     const int lv = (int)min((long long)L, nlines - line0);
-    const float2 *F = Hg + (long long)(6 * h) * g.hstride;
+    const float2 *F = Hg + (long long)(6 * h) * g.hstride + line0 * hp;
+    // the rows of pair s's two fields, asynchronously into the lines' regions of its exchange
+    // (a row is hp complex values, whole 16-byte copies): every load of the block in flight at
+    // once, none held in a register
+    for (int e = 2 * tid; e < lv * hp; e += 2 * (int)blockDim.x) {
+        const int l = (int)fdiv((unsigned)e, g.dhp);
+        const float2 *src = F + e;
+        float2 *d = sm + l * lp + (e - l * hp);
+        col_copy16(d, src);                              // x0
+        col_copy16(d + hp, src + g.hstride);             // y0
+        col_copy16(d + 2 * set, src + 2 * g.hstride);    // z0
+        if (g2) {
+            col_copy16(d + set, src + 3 * g.hstride);
+            col_copy16(d + set + hp, src + 4 * g.hstride);
+            col_copy16(d + 2 * set + hp, src + 5 * g.hstride);
+        }
+    }
+    col_stage_wait();
+    __syncthreads();
     {
         const int l = (int)fdiv((unsigned)tid, lx.dr2), i = tid - l * r2;
-        if (l < lv) {
-            const float2 *r = F + (line0 + l) * g.hp;
-            float2 *d = sm + l * lp + i;
-            const long long hs = g.hstride;
-#define TILD_XI1(R)                                                                                           \
-    do {                                                                                                      \
-        xi_stage1<R>(lx, r, r + hs, true, g.nxh, d, i);                                                       \
-        if (g2) xi_stage1<R>(lx, r + 3 * hs, r + 4 * hs, true, g.nxh, d + set, i);                            \
-        xi_stage1<R>(lx, r + 2 * hs, g2 ? r + 5 * hs : nullptr, false, g.nxh, d + 2 * set, i);                \
+        const bool act = l < lv;
+        float2 *d = sm + l * lp + i;
+#define TILD_XI1(R)                                                                     \
+    do {                                                                                \
+        xi_stage1<R>(lx, d, hp, g.nxh, i, true, true, act);                             \
+        if (g2) xi_stage1<R>(lx, d + set, hp, g.nxh, i, true, true, act);               \
+        xi_stage1<R>(lx, d + 2 * set, hp, g.nxh, i, g2, false, act);                    \
     } while (0)
-            TILD_RADIX(r1, TILD_XI1)
+        TILD_RADIX(r1, TILD_XI1)
 #undef TILD_XI1
-        }
     }
     __syncthreads();
     const int l = (int)fdiv((unsigned)tid, lx.dr1), k1 = tid - l * r1;
@@ -339,13 +382,13 @@ __device__ __forceinline__ void xinv2_body(const Geom &g, const FftLine &lx, int
     }
 }
 
-__global__ void __launch_bounds__(256, 2) k_xinv2(Geom g, FftLine lx, int nfg, const float2 *__restrict__ Hg,
+__global__ void __maxnreg__(96) k_xinv2(Geom g, FftLine lx, int nfg, const float2 *__restrict__ Hg,
                                                   float4 *__restrict__ rec, RecLayout rl, int L)
 {
     xinv2_body(g, lx, nfg, Hg, rec, rl, L, blockIdx.x, blockIdx.y);
 }
 
-__global__ void __launch_bounds__(256, 2) k_xinv2_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre, int R)
+__global__ void __maxnreg__(96) k_xinv2_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre, int R)
 {
     const int r = batch_replica(pre, R, blockIdx.x);
     const BatchRep &b = reps[r];
@@ -353,13 +396,17 @@ __global__ void __launch_bounds__(256, 2) k_xinv2_batch(const BatchRep *__restri
 }
 
 // ---- launch shapes ----
-// Lines (x passes) or columns (y and z passes) per block: 16, whose 128-byte rows are whole
-// cache lines, more on short lines until a block has 128 threads, and 8 where 16 would leave
-// SMs without a block.
-static int lines_of(const FftLine &l, long long nlines, int jobs)
+// Columns (y and z passes) per block: 16, whose 128-byte rows are whole cache lines, more on
+// short lines until a block has 128 threads, and 8 where 16 would leave SMs without a block.
+// Lines (x passes; their rows are contiguous whatever the number): 8 where these already make
+// a block of 112 threads or more (r1 >= 14), since several small blocks per SM overlap their
+// loads and transforms better than two large ones (x inverse, 8 against 16 lines: 192 points
+// 149 and 157 us, 160 points 98 and 110, 75 points 19 and 26; but 100 points, of r1 = 10, 37
+// and 30), else as the columns.
+static int lines_of(const FftLine &l, long long nlines, int jobs, bool rows)
 {
-    int L = 16;
-    while (l.r1 * L < 128) L *= 2;
+    int L = rows && 8 * l.r1 >= 112 ? 8 : 16;
+    while (l.r1 * L < 112) L *= 2;
     while (L > 8 && (nlines + L - 1) / L * jobs < 2 * 148) L /= 2;
     return L;
 }
@@ -371,12 +418,12 @@ static int ilog2(int v)
 }
 static int threads_of(const FftLine &l, int L) { return std::max(64, (std::max(l.r1, l.r2) * L + 31) & ~31); }
 
-int fft2_xfwd_lines(const Geom &g, const FftLine &lx, int npair) { return lines_of(lx, (long long)g.ny * g.nz, npair); }
+int fft2_xfwd_lines(const Geom &g, const FftLine &lx, int npair) { return lines_of(lx, (long long)g.ny * g.nz, npair, true); }
 int fft2_xinv_lines(const Geom &g, const FftLine &lx, int nfg)
 {
-    return std::min(16, lines_of(lx, (long long)g.ny * g.nz, (nfg + 1) / 2));   // three exchanges per line
+    return std::min(16, lines_of(lx, (long long)g.ny * g.nz, (nfg + 1) / 2, true));   // three exchanges per line
 }
-int fft2_col_bits(const FftLine &l, long long ncols, int jobs) { return ilog2(lines_of(l, ncols, jobs)); }
+int fft2_col_bits(const FftLine &l, long long ncols, int jobs) { return ilog2(lines_of(l, ncols, jobs, false)); }
 
 void fft2_shape(int stage, const Geom &g, const FftLine &l, int n, int L, int *bx, int *by, int *threads, size_t *smem)
 {
@@ -398,7 +445,7 @@ void fft2_shape(int stage, const Geom &g, const FftLine &l, int n, int L, int *b
             break;
         default:        // BS_XINV
             *by = (n + 1) / 2;
-            *smem = 3 * (size_t)L * x_pitch(l.r1, l.r2) * sizeof(float2);
+            *smem = 3 * (size_t)L * xi_pitch(l.r1, l.r2, g.hp) * sizeof(float2);
             break;
     }
 }

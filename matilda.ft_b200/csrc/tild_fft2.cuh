@@ -51,9 +51,26 @@ __device__ __forceinline__ void stage1_reg(float2 *v, const float2 *__restrict__
     }
 }
 
-// ---- column passes: C = 1 << cb lines side by side, element (k1, i) of column c at
-// ((k1 r2 + i) << cb) + c: consecutive threads on consecutive columns, no bank conflicts
-// (a half warp covers 16 consecutive complex values) ----
+// ---- column passes: C = 1 << cb lines side by side, element t of column c at (t << cb) + c:
+// consecutive threads on consecutive columns, no bank conflicts (a half warp covers 16
+// consecutive complex values).  Both stages work in place: the first stage's thread i reads
+// the elements i + r2 q and writes (k1, i) to element k1 r2 + i, the same places, and the
+// second stage's thread k1 reads its row.  So the columns arrive by 16-byte asynchronous
+// copies straight into the exchange, all in flight at once and none held in a register. ----
+__device__ __forceinline__ void col_copy16(float2 *dst, const float2 *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+// rows of this thread's column pair cc (even), n rows of pitch `pitch` (even) from src
+__device__ __forceinline__ void col_stage(float2 *S, const float2 *src, long long pitch, int n, int cb, int cc)
+{
+    const int step = (int)blockDim.x >> (cb - 1);
+    for (int t = (int)threadIdx.x >> (cb - 1); t < n; t += step) col_copy16(S + (t << cb) + cc, src + t * pitch);
+}
+__device__ __forceinline__ void col_stage_wait()
+{
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+}
 template <int R>
 __device__ __forceinline__ void col_load(float2 *v, const float2 *__restrict__ s, int pitch)
 {
