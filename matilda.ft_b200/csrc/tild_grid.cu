@@ -166,6 +166,30 @@ __device__ __forceinline__ void global_add(float2 *dep, unsigned long long *depf
     else atomicAdd(FIELD_PTR(dep, f, M) + 2 * m, v);
 }
 
+// All points of one particle into an int32 box: c0 (carrying the tile's fixed-point scale)
+// into b0, and into b1 nothing (MODE 0), sg (0 or +-1) times the same value (MODE 1: one
+// conversion for both fields, an addition of 0 rather than a branch per point) or c1's own
+// (MODE 2).  The coefficient is folded into Wy Wz: for c0 = +-1 the same bits as folding it last.
+template <int P, int MODE>
+__device__ __forceinline__ void deposit_points(int *b0, int *b1, int E0, int E01, const float *Wx, const float *Wy,
+                                               const float *Wz, float c0, float c1, int sg)
+{
+#pragma unroll
+    for (int e = 0; e <= P; e++)
+#pragma unroll
+        for (int b = 0; b <= P; b++) {
+            const float w = Wy[b] * Wz[e], w0 = w * c0, w1 = w * c1;
+            const int r = e * E01 + b * E0;
+#pragma unroll
+            for (int a = 0; a <= P; a++) {
+                const int k = __float2int_rn(Wx[a] * w0);
+                atomicAdd(b0 + r + a, k);
+                if (MODE == 1) atomicAdd(b1 + r + a, k * sg);
+                if (MODE == 2) atomicAdd(b1 + r + a, __float2int_rn(Wx[a] * w1));
+            }
+        }
+}
+
 // Deposit of one tile of sorted particles (or a window of slots).  The box of grid points
 // is accumulated in shared memory, each thread adding its particle's (P+1)^3 points with
 // shared-memory atomics (the atomics have throughput to spare; what bounds the deposit
@@ -277,6 +301,22 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
                     for (int f = 0; f < NC; f++) cf[f] = f < nfields ? field_coef(dm, dq, f, qp) : 0.f;
                 }
             }
+            if constexpr (!FIXED && NF >= 1) {
+                if (ia) {   // (uniform over the CTA)
+                    const int first = cf[0] != 0.f ? 0 : 1;
+                    const float ca = NF == 2 && first ? cf[NF - 1] : cf[0], cb = NF == 2 && !first ? cf[NF - 1] : 0.f;
+                    const int sg = cb == 0.f ? 0 : (cb == ca ? 1 : (cb == -ca ? -1 : 2));
+                    const bool second = __any_sync(full, sg != 0), other = __any_sync(full, sg == 2);
+                    if (ca != 0.f) {
+                        int *w0 = reinterpret_cast<int *>(smraw) + o + (NF == 2 ? first * V : 0), *w1 = reinterpret_cast<int *>(smraw) + o + V;
+                        if (NF == 1 || !second) deposit_points<P, 0>(w0, w1, E0, E01, Wx, Wy, Wz, ca * tfix, 0.f, 0);
+                        else if (!other) deposit_points<P, 1>(w0, w1, E0, E01, Wx, Wy, Wz, ca * tfix, 0.f, sg);
+                        else deposit_points<P, 2>(w0, w1, E0, E01, Wx, Wy, Wz, ca * tfix, cb * tfix, sg);
+                    }
+                    __syncwarp();
+                    continue;
+                }
+            }
             float c0 = 0.f;
             int sgn[NC];
             bool general = false;
@@ -313,11 +353,12 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
                     }
             };
             // the box's number type is fixed for the tile, the conversion per warp
+            constexpr bool IB = !FIXED && NF == 0;   // int32 boxes of one or two fields: above
             if (__any_sync(full, general)) {
-                if (ia) points(std::true_type{}, std::true_type{});
+                if (IB && ia) points(std::integral_constant<bool, IB>{}, std::true_type{});
                 else points(std::false_type{}, std::true_type{});
             } else {
-                if (ia) points(std::true_type{}, std::false_type{});
+                if (IB && ia) points(std::integral_constant<bool, IB>{}, std::false_type{});
                 else points(std::false_type{}, std::false_type{});
             }
         }
@@ -374,9 +415,7 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
                     a0 = (float)__float_as_int(a0) * tinv;
                     a1 = (float)__float_as_int(a1) * tinv;
                 }
-                if (a0 != 0.f && a1 != 0.f) atomicAdd(dep + t * g.M + m, make_float2(a0, a1));
-                else if (a0 != 0.f) atomicAdd(&dep[t * g.M + m].x, a0);
-                else if (a1 != 0.f) atomicAdd(&dep[t * g.M + m].y, a1);
+                if (a0 != 0.f || a1 != 0.f) atomicAdd(dep + t * g.M + m, make_float2(a0, a1));
             }
         }
     });
