@@ -166,6 +166,40 @@ __device__ __forceinline__ void global_add(float2 *dep, unsigned long long *depf
     else atomicAdd(FIELD_PTR(dep, f, M) + 2 * m, v);
 }
 
+// The deterministic mode's 2^32 fixed-point contributions as two int32 words per point and
+// field, the low 16 bits and the rest: the flush adds (hi << 16) + lo, the same integer sum.
+// 64-bit shared-memory additions run as compare-and-swap loops, some ten times slower than
+// int32 ones (three fields, 200,000 particles: 141 -> 50 us); two words are exact while the hi
+// and lo sums stay inside int32: up to 32767 particles per tile, and 256 times the fast mode's
+// count bound.  Tiles beyond that keep the 64-bit box.
+template <int P, int NF>
+__device__ __forceinline__ void deposit_points_split(int *b0, int V, int E0, int E01, const float *Wx, const float *Wy,
+                                                     const float *Wz, const float *cf)
+{
+#pragma unroll 1
+    for (int f = 0; f < NF; f++) {
+        const float c = sel<NF - 1>(cf, f);
+        if (c == 0.f) continue;
+        int *bf = b0 + 2 * f * V;
+#pragma unroll 1
+        for (int e = 0; e <= P; e++) {
+            const float wz = sel<P>(Wz, e);
+#pragma unroll
+            for (int b = 0; b <= P; b++) {
+                const float w = Wy[b] * wz;
+                int *r = bf + e * E01 + b * E0;
+#pragma unroll
+                for (int a = 0; a <= P; a++) {
+                    // c w 2^32: the product with the power of two is exact
+                    const long long k = __float2ll_rn(__fmul_rn(__fmul_rn(c, __fmul_rn(Wx[a], w)), 4294967296.f));
+                    atomicAdd(r + a, (int)(k & 0xffff));
+                    atomicAdd(r + a + V, (int)(k >> 16));
+                }
+            }
+        }
+    }
+}
+
 // All points of one particle into an int32 box: c0 (carrying the tile's fixed-point scale)
 // into b0, and into b1 nothing (MODE 0), sg (0 or +-1) times the same value (MODE 1: one
 // conversion for both fields, an addition of 0 rather than a branch per point) or c1's own
@@ -229,6 +263,8 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
     int ksh = 0;
     while (ksh < kTileFixSteps && (long long)(b1 - b0) > ((long long)int_tile_max << ksh)) ksh++;
     const bool ia = !FIXED && staged && (long long)(b1 - b0) <= ((long long)int_tile_max << ksh);
+    // deterministic mode: two int32 words per point and field (see deposit_points_split)
+    const bool split = FIXED && staged && b1 - b0 <= 32767 && (long long)(b1 - b0) <= ((long long)int_tile_max << 8);
     const float tfix = __int_as_float((127 + kTileFixLog2 - ksh) << 23);      // 2^(24 - k)
     const float tinv = __int_as_float((127 - kTileFixLog2 + ksh) << 23);      // 2^-(24 - k)
     float *tf = reinterpret_cast<float *>(smraw);
@@ -314,6 +350,12 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
                         else deposit_points<P, 2>(w0, w1, E0, E01, Wx, Wy, Wz, ca * tfix, cb * tfix, sg);
                     }
                     __syncwarp();
+                    continue;
+                }
+            }
+            if constexpr (FIXED) {
+                if (split) {
+                    if (dm) deposit_points_split<P, NC>(reinterpret_cast<int *>(smraw) + o, V, E0, E01, Wx, Wy, Wz, cf);
                     continue;
                 }
             }
@@ -404,7 +446,13 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
     tile_for_each(ts, E, E[0], E[0] * E[1], [&](int v, int m) {
         if (FIXED) {
             for (int f = 0; f < nfields; f++) {
-                const unsigned long long u = tu[f * V + v];
+                unsigned long long u;
+                if (split) {
+                    const int *w = reinterpret_cast<const int *>(smraw) + 2 * f * V + v;
+                    u = (unsigned long long)(((long long)w[V] << 16) + w[0]);
+                } else {
+                    u = tu[f * V + v];
+                }
                 if (u) atomicAdd(depfix + f * g.M + m, u);
             }
         } else {
