@@ -2304,24 +2304,28 @@ void Box::getDensity(const std::string &group, int charge, float *rho)
     if (!ready) fail(TILD_ERR_STATE, "endBox has not been processed");
     const int gi = findGroupInteger(group);
     if (charge && !psGroup[gi].isCharges) fail(TILD_ERR_ARG, "only the 'charges' group has a charge density");
+    ck(cudaSetDevice(device), "cudaSetDevice");
+    float *dRho = groupDensity(gi, charge);
+    ck(cudaMemcpyAsync(rho, dRho, 4 * geom.M, cudaMemcpyDeviceToHost, stream), "read density");
+    ck(cudaStreamSynchronize(stream), "density");
+}
+
+// A group's density (or charge density) at the current positions with the reference's weights,
+// deposited on the box's stream into scratch the box owns: the gradient half spectra, which no
+// call reads once the step or force evaluation that made them is over (3 nfg hstride complex
+// values, at least 1.5 M), and the site slots in the position scratch.  (Allocating and freeing
+// device memory on each call took most of a density or structure-factor call's time.)
+float *Box::groupDensity(int gi, int charge)
+{
+    const std::vector<int> &sites = psGroup[gi].siteList;
+    float *dRho = reinterpret_cast<float *>(dHg);
+    int *dSlotOf = reinterpret_cast<int *>(dTmp), *dSites = dSlotOf + nstot;
     const long long s = deviceStep();
-    const std::vector<int> orig = slotOrder();
-    std::vector<int> slotOf(nstot);
-    for (int64_t k = 0; k < nstot; k++) slotOf[orig[k]] = (int)k;
-    std::vector<int> sites(psGroup[gi].siteList);
-    for (int &v : sites) v = slotOf[v];
-    int *dSites = nullptr;
-    float *dRho = nullptr;
-    ck(cudaMalloc(&dSites, 4 * sites.size()), "malloc");
-    ck(cudaMalloc(&dRho, 4 * geom.M), "malloc");
-    cudaMemcpy(dSites, sites.data(), 4 * sites.size(), cudaMemcpyHostToDevice);
-    cudaMemset(dRho, 0, 4 * geom.M);
-    cudaError_t e = launch_density_single(geom, ppHost, dX[s & 1], dSites, (int)sites.size(), dQ, charge, dRho, stream);
-    cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) e = cudaMemcpy(rho, dRho, 4 * geom.M, cudaMemcpyDeviceToHost);
-    cudaFree(dSites);
-    cudaFree(dRho);
-    ck(e, "density");
+    ck(cudaMemsetAsync(dRho, 0, 4 * geom.M, stream), "clear density");
+    ck(cudaMemcpyAsync(dSites, sites.data(), 4 * sites.size(), cudaMemcpyHostToDevice, stream), "copy sites");
+    ck(launch_slot_map(dOrig, (int)nstot, dSlotOf, dSites, (int)sites.size(), stream), "slot map");
+    ck(launch_density_single(geom, ppHost, dX[s & 1], dSites, (int)sites.size(), dQ, charge, dRho, stream), "density");
+    return dRho;
 }
 
 // Grid force of a group from the last force evaluation (tild_box_forces or a step), in the
@@ -2419,40 +2423,23 @@ void Box::structureFactor(const std::string &group, int charge, int nbins, doubl
     const int gi = findGroupInteger(group);
     if (charge && !psGroup[gi].isCharges) fail(TILD_ERR_ARG, "only the 'charges' group has a charge density");
     ck(cudaSetDevice(device), "cudaSetDevice");
-    const long long s = deviceStep();
-    const std::vector<int> orig = slotOrder();
-    std::vector<int> slotOf(nstot);
-    for (int64_t k = 0; k < nstot; k++) slotOf[orig[k]] = (int)k;
-    std::vector<int> sites(psGroup[gi].siteList);
-    for (int &v : sites) v = slotOf[v];
     const Geom &g = geom;
-    int *dSites = nullptr;
-    float *dRho = nullptr;
-    float2 *dPair = nullptr, *dHs = nullptr;
-    double *dBins = nullptr;
-    cudaError_t e = cudaMalloc(&dSites, 4 * std::max<size_t>(1, sites.size()));
-    if (e == cudaSuccess) e = cudaMalloc(&dRho, 4 * g.M);
-    if (e == cudaSuccess) e = cudaMalloc(&dPair, 8 * g.M);
-    if (e == cudaSuccess) e = cudaMalloc(&dHs, 8 * g.hstride);
-    if (e == cudaSuccess) e = cudaMalloc(&dBins, 3 * sizeof(double) * nbins);
-    if (e == cudaSuccess && !sites.empty())
-        e = cudaMemcpy(dSites, sites.data(), 4 * sites.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dRho, 0, 4 * g.M, stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(dBins, 0, 3 * sizeof(double) * nbins, stream);
-    if (e == cudaSuccess)
-        e = launch_density_single(g, ppHost, dX[s & 1], dSites, (int)sites.size(), dQ, charge, dRho, stream);
-    if (e == cudaSuccess) e = launch_to_pairs(dRho, dPair, g.M, stream);
-    if (e == cudaSuccess)
-        e = launch_structure_factor(g, lx, ly, lz, ksHost.twopi_over_L, dPair, dHs, nbins, kmax / nbins, dBins, stream);
+    if (binCap < nbins) {   // kept for later calls, doubled when a call asks for more
+        const int cap = std::max(256, std::max(nbins, 2 * binCap));
+        dBins = dalloc<double>(3 * (size_t)cap);
+        binCap = cap;
+    }
+    float *dRho = groupDensity(gi, charge);
+    // the packed pairs after the density in the gradient half spectra (M/2 + 2 + M complex
+    // values of at least 1.5 M + 3 ny nz), the spectrum in the density half spectra
+    float2 *dPair = dHg + ((g.M + 3) / 4) * 2;
+    ck(cudaMemsetAsync(dBins, 0, 3 * sizeof(double) * nbins, stream), "clear bins");
+    ck(launch_to_pairs(dRho, dPair, g.M, stream), "structure factor");
+    ck(launch_structure_factor(g, lx, ly, lz, ksHost.twopi_over_L, dPair, dH, nbins, kmax / nbins, dBins, stream),
+       "structure factor");
     std::vector<double> b(3 * (size_t)nbins, 0.0);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-    if (e == cudaSuccess) e = cudaMemcpy(b.data(), dBins, 3 * sizeof(double) * nbins, cudaMemcpyDeviceToHost);
-    cudaFree(dSites);
-    cudaFree(dRho);
-    cudaFree(dPair);
-    cudaFree(dHs);
-    cudaFree(dBins);
-    ck(e, "structure factor");
+    ck(cudaMemcpyAsync(b.data(), dBins, 3 * sizeof(double) * nbins, cudaMemcpyDeviceToHost, stream), "structure factor");
+    ck(cudaStreamSynchronize(stream), "structure factor");
     for (int i = 0; i < nbins; i++) {
         const double n = b[3 * i + 2];
         if (sk_out) sk_out[i] = n > 0.0 ? b[3 * i] / n : 0.0;

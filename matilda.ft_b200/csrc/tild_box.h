@@ -151,6 +151,7 @@ private:
     void buildPlan();
     void allocDevice();
     void planTransforms();
+    float *groupDensity(int gi, int charge);   // into scratch, on the box's stream
     void forwardXY();
     void freeDevice();
     void uploadParticles();
@@ -274,6 +275,8 @@ private:
     float *dUk = nullptr;   // FP32 û(k) shape table, one half-spectrum field per potential
     ParticleParams *dPp = nullptr;
     double *dEpart = nullptr, *dBpart = nullptr, *dRes = nullptr;
+    double *dBins = nullptr;        // structure-factor shells (3 per shell), kept between calls
+    int binCap = 0;
     KSpace *hKsPinned = nullptr;
     cudaGraphExec_t gNorm = nullptr, gEnergy = nullptr;
     std::vector<double> stageSec;
