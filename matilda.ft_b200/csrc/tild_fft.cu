@@ -52,20 +52,21 @@ __device__ __forceinline__ void fft_stage(const float2 *__restrict__ src, float2
     }
 }
 
-// Generic radix stage: b_q = sum_s a_s W_{pR}^{s k} W_R^{q s}, R an odd prime (11, 13,
-// ...: the plan takes 2, 3, 5 and 7 first).  One thread per output pair (q, R - q) of a
-// butterfly, so that a prime line (one butterfly of radix n) still spreads over (n+1)/2
-// threads: W_R^{(R-q) s} = conj W_R^{q s}, so both outputs share each term's loads and
-// products; each sums its R terms in order s = 0..R-1.
+// Generic radix stage, R an odd prime (17, 19, ...: the plan takes 2, 3, 5 and 7 first, and the
+// smaller primes of short lines run in two register stages).  With the twiddled inputs a_s,
+// t_s = a_s + a_{R-s} and u_s = a_s - a_{R-s} (s <= (R-1)/2), the output pair (q, R - q) is
+// m_q -+ i n_q with m_q = a_0 + sum_s cos(2 pi q s/R) t_s and n_q = sum_s sin(2 pi q s/R) u_s.
+// A first sweep leaves t_s and u_s in the places of a_s and a_{R-s}; then one thread per output
+// pair of a butterfly, so that a prime line (one butterfly of radix n) still spreads over
+// (n+1)/2 threads, takes two packed FMAs and three shared loads for every two inputs.  (Summing
+// R products per output pair took about 3.5 times the instructions.)
 template <bool INV>
-__device__ void fft_stage_generic(const float2 *__restrict__ src, float2 *__restrict__ dst, int L, int lp, int ls,
+__device__ void fft_stage_generic(float2 *__restrict__ src, float2 *__restrict__ dst, int L, int lp, int ls,
                                   int n, int R, int p, const FastDiv &dp, const FastDiv &dsplit, bool line_fast,
                                   const float2 *tw)
 {
-    const int nb = n / R, stride = n / (p * R), nR = n / R, items = L * nb, half = (R + 1) / 2;
-    for (int w = threadIdx.x; w < items * half; w += blockDim.x) {
-        const int qq = w / items, wi = w - qq * items;
-        int l, i;
+    const int nb = n / R, stride = n / (p * R), items = L * nb, half = (R + 1) / 2, sb = nb * ls;
+    auto place = [&](int wi, int &l, int &i) {
         if (line_fast) {
             i = (int)fdiv((unsigned)wi, dsplit);
             l = wi - i * L;
@@ -73,30 +74,45 @@ __device__ void fft_stage_generic(const float2 *__restrict__ src, float2 *__rest
             l = (int)fdiv((unsigned)wi, dsplit);
             i = wi - l * nb;
         }
+    };
+    for (int w = threadIdx.x; w < items * (half - 1); w += blockDim.x) {
+        const int s = w / items + 1, wi = w - (s - 1) * items;
+        int l, i;
+        place(wi, l, i);
         const int k = i - p * (int)fdiv((unsigned)i, dp);
-        const float2 *s = src + l * lp;
-        const int j = (i - k) * R + k;
-        float2 acc = make_float2(0.f, 0.f), acm = make_float2(0.f, 0.f);   // b_q, b_{R-q}
-        int e = 0;   // (qq * ss) mod R
-        for (int ss = 0; ss < R; ss++) {
-            float2 v = s[(i + ss * nb) * ls];
-            if (k && ss) v = cmul(v, twid<INV>(tw, ss * k * stride));
-            if (e) {
-                const float2 t = twid<INV>(tw, e * nR);
-                const float xr = v.x * t.x, yi = v.y * t.y, xi = v.x * t.y, yr = v.y * t.x;
-                acc.x += xr - yi;
-                acc.y += xi + yr;
-                acm.x += xr + yi;
-                acm.y += yr - xi;
-            } else {
-                acc = cadd(acc, v);
-                acm = cadd(acm, v);
-            }
-            e += qq;
-            if (e >= R) e -= R;
+        float2 *e = src + l * lp + i * ls;
+        float2 a = e[s * sb], b = e[(R - s) * sb];
+        if (k) {
+            a = cmul(a, twid<INV>(tw, s * k * stride));
+            b = cmul(b, twid<INV>(tw, (R - s) * k * stride));
         }
-        dst[l * lp + (j + qq * p) * ls] = acc;
-        if (qq) dst[l * lp + (j + (R - qq) * p) * ls] = acm;
+        e[s * sb] = cadd(a, b);
+        e[(R - s) * sb] = csub(a, b);
+    }
+    __syncthreads();
+    for (int w = threadIdx.x; w < items * half; w += blockDim.x) {
+        const int q = w / items, wi = w - q * items;
+        int l, i;
+        place(wi, l, i);
+        const int k = i - p * (int)fdiv((unsigned)i, dp);
+        const float2 *e = src + l * lp + i * ls;
+        float2 *o = dst + l * lp + ((i - k) * R + k) * ls;
+        float2 m = e[0], v = make_float2(0.f, 0.f);
+        const float2 *t = e, *u = e + R * sb;
+        int x = 0;   // (q s) mod R
+#pragma unroll 4
+        for (int s = 1; s < half; s++) {
+            t += sb;
+            u -= sb;
+            x += q;
+            if (x >= R) x -= R;
+            const float2 c = tw[x * nb];   // cos, -sin
+            m = cfma(c.x, *t, m);
+            v = cfma(-c.y, *u, v);
+        }
+        const float2 iv = INV ? mul_pi(v) : mul_mi(v);
+        o[q * p * ls] = cadd(m, iv);
+        if (q) o[(R - q) * p * ls] = csub(m, iv);
     }
 }
 
