@@ -40,8 +40,8 @@ METRIC = "particle-steps/s"
 WORKLOAD = ("c2_coacervate: 2,097,152 particles, 192^3 grid, pmeorder 3, gaussian(all,all) + "
             "smeared charges (lB 1.0, sigma 0.5), harmonic bonds, GJF dt 0.005")
 STAGES = ["deposit", "fft_x_fwd", "fft_y_fwd", "kspace_z", "fft_y_inv", "fft_x_inv", "gather", "integrate"]
-KERNEL_NAMES = {"deposit": "k_deposit", "fft_x_fwd": "k_xfwd", "fft_y_fwd": "k_ypass<false>",
-                "kspace_z": "k_kspace_z", "fft_y_inv": "k_ypass<true>", "fft_x_inv": "k_xinv",
+KERNEL_NAMES = {"deposit": "k_deposit", "fft_x_fwd": "k_xfwd2", "fft_y_fwd": "k_ypass2<false>",
+                "kspace_z": "k_kspace2", "fft_y_inv": "k_ypass2<true>", "fft_x_inv": "k_xinv2",
                 "gather": "k_gather_paired", "integrate": "k_integrate"}
 KERNELS_PER_STEP = 9   # deposit, xfwd, yfwd, kspace_z, yinv, xinv, gather, integrate, tick
 
@@ -65,10 +65,12 @@ def algorithmic_bytes(spec, nd=2, nfg=2, maxb=2, charged=True):
     qb = 4 if charged else 0
     return {
         "deposit": N * (12 + 4 + qb) + npair * M * 8,
-        "fft_x_fwd": npair * M * 8 + nd * hs,
+        # the deposit target read and cleared for the next step
+        "fft_x_fwd": 2 * npair * M * 8 + nd * hs,
         "fft_y_fwd": 2 * nd * hs,
-        "kspace_z": nd * hs + 3 * nfg * hs,
-        "fft_y_inv": 2 * 3 * nfg * hs,
+        # two fields per force group out of the z pass, the third made by the y pass
+        "kspace_z": nd * hs + 2 * nfg * hs,
+        "fft_y_inv": 2 * nfg * hs + 3 * nfg * hs,
         # the force records: paired planes, 12 bytes per point and force group
         "fft_x_inv": 3 * nfg * hs + nfg * M * 12,
         # x_t 12, flags 4, q, the grid force written 12, the records read once

@@ -301,11 +301,12 @@ int tild_pool_stats(tild_pool *pool, int64_t *out, int32_t nout);
  * same pmeorder, one or two density fields and force groups in each, the same
  * deterministic mode and sort_interval, no ramped potential, and the tile gather (sorted
  * tiles with TMA boxes).  Sizes, grids, potentials' amplitudes, tiles, integrators and
- * seeds may differ.  Each step runs every stage of the TILD step (zeroing the deposit
- * targets, the deposit, the five transform passes, the grid gather, the integrator pass,
- * the step counters) as ONE kernel launch over the work of all replicas -- their
- * geometries, FFT plans, tile lists and TMA descriptors in a device table -- and the ten
- * launches of a step are captured once in a CUDA graph; each replica's spatial re-sort
+ * seeds may differ.  Each step runs every stage of the TILD step (the deposit, the five
+ * transform passes, the grid gather, the integrator pass, the step counters) as ONE kernel
+ * launch over the work of all replicas -- their geometries, FFT plans, tile lists and TMA
+ * descriptors in a device table; a transform pass takes a second launch where some replicas'
+ * grids run in two register stages and others' in mixed radices -- and the launches of a
+ * step are captured once in a CUDA graph; each replica's spatial re-sort
  * runs every sort_interval steps as a branch of one more graph.  A step is bit-identical to
  * tild_box_step on each replica in deterministic mode.  The boxes stay the caller's: read
  * them with tild_box_get_positions, tild_box_thermo and the like; destroy the batch before
