@@ -100,6 +100,7 @@ void Batch::build()
     const int R = (int)boxes.size();
     if (R == 0) return;
     cudaSetDevice(device);
+    init_fft_batch_attributes();
     auto maxPrime = [](int n) {
         int m = n, p = 1;
         for (int f = 2; f * f <= m; f++)

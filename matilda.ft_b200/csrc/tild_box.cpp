@@ -993,7 +993,6 @@ void Box::initDevice()
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
         ownStream = true;
     }
-    init_fft_attributes();
     init_deposit_attributes();
     init_particle_attributes();
     allocDevice();
@@ -1318,6 +1317,8 @@ void Box::planTransforms()
     const int nd = (int)dfields.size(), nfg = (int)fgroups.size();
     twoStage = fft_two_stage(lx, ly, lz, nd, nfg);
     nblkZ = kspace_blocks(geom, lz, nd, nfg, (int)potentials.size(), twoStage);
+    if (twoStage) init_fft2_attributes(nd);   // only the kernels this box launches: each call costs set-up time
+    else init_fft_attributes();
 }
 
 void Box::uploadParticles()

@@ -308,8 +308,11 @@ void kspace2_shape(const Geom &g, const FftLine &lz, int nf, int cb, int *blocks
 cudaError_t launch_fft2_batch(int stage, const BatchRep *reps, int R, const BatchLaunch &bl, int deterministic,
                               cudaStream_t st);
 cudaError_t launch_kspace2_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int nf, cudaStream_t st);
-void init_fft2_attributes();
-void init_kspace2_attributes();
+void init_fft2_attributes(int nf);         // large dynamic shared memory, for boxes of nf fields
+void init_kspace2_attributes(int nf);
+void init_fft2_batch_attributes();         // and for batches
+void init_kspace2_batch_attributes();
+void init_fft_batch_attributes();
 // fills ks.cm from its terms and the potentials' amplitudes
 void kspace2_coefficients(KSpace &ks);
 // blocks of the k-space pass over one box (the rows of its energy partials)

@@ -678,6 +678,11 @@ void init_fft_attributes()
     set_max_smem(k_kspace_z<2>, kKspaceSmemMax);
     set_max_smem(k_sk_z<kTXz>, 200 * 1024);
     set_max_smem(k_xinv, 200 * 1024);
+}
+
+void init_fft_batch_attributes()
+{
+    init_fft2_batch_attributes();
     set_max_smem(k_xfwd_batch<true>, 200 * 1024);
     set_max_smem(k_xfwd_batch<false>, 200 * 1024);
     set_max_smem(k_ypass_batch<false, kTXy>, 200 * 1024);
@@ -685,8 +690,6 @@ void init_fft_attributes()
     set_max_smem(k_kspace_batch<4>, kKspaceSmemMax);
     set_max_smem(k_kspace_batch<2>, kKspaceSmemMax);
     set_max_smem(k_xinv_batch, 200 * 1024);
-    init_fft2_attributes();
-    init_kspace2_attributes();
 }
 
 void build_fft_line(int n, double twopi_over_L, FftLine &pl, float2 *dev)

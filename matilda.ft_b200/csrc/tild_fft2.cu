@@ -10,7 +10,8 @@ namespace tild {
 // A(k) = (Z(k) + conj Z(n-k))/2 and B(k) = (Z(k) - conj Z(n-k))/(2i), k in [0, n/2].  A
 // block takes L lines of one pair; a line's exchange pitch lp = r2 (mod 16) puts the
 // consecutive threads (l, i) of the first stage on consecutive complex values.  The rows
-// are the block's alone, so it also clears them for the next step's deposit.
+// are the block's alone, so it also clears them for the next step's deposit.  Bound by the
+// latency of the row loads (192^3, one pair: 51 us and a memset of 10 us -> 37 us, 170 MB).
 // -------------------------------------------------------------------------------------
 template <int R1, bool FIXED>
 __device__ __forceinline__ void xf_stage1(const FftLine &lx, float2 *E, int lp, int l, int i, long long row, long long M,
@@ -133,7 +134,9 @@ __global__ void __launch_bounds__(256, 3) k_xfwd2_batch(const BatchRep *__restri
 
 // -------------------------------------------------------------------------------------
 // y-axis passes over C columns: column j of a field is (z, kx) = (j / hp, j mod hp), so the
-// blocks tile nz hp columns without a remainder per plane.
+// blocks tile nz hp columns without a remainder per plane.  Bound by load latency between
+// the barriers, at four blocks of 64 registers per SM (192^3: two fields forward 43 -> 31 us,
+// six gradient fields inverse 109 -> 80 us, 286 MB where the pass before read 343).
 // -------------------------------------------------------------------------------------
 template <bool INV, int R1, bool GRAD>
 __device__ __forceinline__ void y_stage1(const FftLine &ly, float2 *d, int set, int cb, int i, bool grad)
@@ -226,7 +229,9 @@ __global__ void __launch_bounds__(256, 4) k_ypass2_batch(const BatchRep *__restr
 // line, (x, y) of each group and (z, z) of both, the Hermitian completion done as the first
 // stage loads (the upper half of a line is the conjugate of the lower one read backwards).
 // Fields 3f hold phi_f after the y pass: times -i k_x here.  A thread of the second stage
-// ends with r2 points of all three pairs, so the records go out as whole float4/float2.
+// ends with r2 points of two pairs at a time, so the records go out as whole float4/float2.
+// Bound by the three exchanges per line that limit an SM to five blocks of 128 threads
+// (192^3: 211 -> 116 us, 342 MB; with the rows loaded through registers 149).
 // -------------------------------------------------------------------------------------
 // First stage of a pair's lines in place: a and b are the staged rows of the two fields in the
 // line's region of the exchange, d its element (0, i); every thread of the block reaches the
@@ -450,19 +455,20 @@ void fft2_shape(int stage, const Geom &g, const FftLine &l, int n, int L, int *b
     }
 }
 
-void init_fft2_attributes()
+// the kernels whose exchanges pass 48 KB (the forward passes' never do)
+void init_fft2_attributes(int nf)
 {
     auto big = [](auto *fn) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); };
-    big(k_xfwd2<true>);
-    big(k_xfwd2<false>);
     big(k_ypass2<true>);
-    big(k_ypass2<false>);
     big(k_xinv2);
-    big(k_xfwd2_batch<true>);
-    big(k_xfwd2_batch<false>);
+    init_kspace2_attributes(nf);
+}
+void init_fft2_batch_attributes()
+{
+    auto big = [](auto *fn) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024); };
     big(k_ypass2_batch<true>);
-    big(k_ypass2_batch<false>);
     big(k_xinv2_batch);
+    init_kspace2_batch_attributes();
 }
 
 cudaError_t launch_xfwd2(const Geom &g, const FftLine &lx, int nd, float2 *dep, unsigned long long *dep_fixed, float2 *H,

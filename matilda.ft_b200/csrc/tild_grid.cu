@@ -204,6 +204,9 @@ __device__ __forceinline__ void deposit_points_split(int *b0, int V, int E0, int
 // into b0, and into b1 nothing (MODE 0), sg (0 or +-1) times the same value (MODE 1: one
 // conversion for both fields, an addition of 0 rather than a branch per point) or c1's own
 // (MODE 2).  The coefficient is folded into Wy Wz: for c0 = +-1 the same bits as folding it last.
+// About 4 instructions per atomic instead of 18 (160^3 diblock melt, one field per particle:
+// 138 -> 92 us); with two fields on every particle the shared atomics' bank conflicts bound it
+// (192^3 coacervate, 89 % of the L1 pipe: 174 -> 164 us).
 template <int P, int MODE>
 __device__ __forceinline__ void deposit_points(int *b0, int *b1, int E0, int E01, const float *Wx, const float *Wy,
                                                const float *Wz, float c0, float c1, int sg)

@@ -13,6 +13,8 @@ template <int NF>
 cudaError_t kspace2_launch_batch(const BatchRep *reps, int R, const BatchLaunch &bl, cudaStream_t st);
 template <int NF>
 void kspace2_attributes(int smem);
+template <int NF>
+void kspace2_batch_attributes(int smem);
 
 // ---- launch shapes ----
 constexpr size_t kKspace2SmemMax = 220 * 1024;
@@ -45,12 +47,20 @@ void kspace2_coefficients(KSpace &ks)
     }
 }
 
-void init_kspace2_attributes()
+void init_kspace2_attributes(int nf)
 {
-    kspace2_attributes<1>((int)kKspace2SmemMax);
-    kspace2_attributes<2>((int)kKspace2SmemMax);
-    kspace2_attributes<3>((int)kKspace2SmemMax);
-    kspace2_attributes<4>((int)kKspace2SmemMax);
+    const int smem = (int)kKspace2SmemMax;
+    switch (nf) {
+        case 1: kspace2_attributes<1>(smem); break;
+        case 2: kspace2_attributes<2>(smem); break;
+        case 3: kspace2_attributes<3>(smem); break;
+        default: kspace2_attributes<4>(smem); break;
+    }
+}
+void init_kspace2_batch_attributes()
+{
+    kspace2_batch_attributes<1>((int)kKspace2SmemMax);
+    kspace2_batch_attributes<2>((int)kKspace2SmemMax);
 }
 
 cudaError_t launch_kspace2(const Geom &g, const FftLine &lz, const KSpace &ks, const KSpace *ks_dev, const float2 *H,

@@ -274,6 +274,8 @@ template <int NF>
 cudaError_t kspace2_launch_batch(const BatchRep *reps, int R, const BatchLaunch &bl, cudaStream_t st);
 template <int NF>
 void kspace2_attributes(int smem);
+template <int NF>
+void kspace2_batch_attributes(int smem);
 
 #ifdef TILD_KSPACE2_NF
 template <>
@@ -290,11 +292,13 @@ void kspace2_attributes<TILD_KSPACE2_NF>(int smem)
 {
     cudaFuncSetAttribute(k_kspace2<TILD_KSPACE2_NF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     cudaFuncSetAttribute(k_kspace2<TILD_KSPACE2_NF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-#if TILD_KSPACE2_NF <= 2
-    cudaFuncSetAttribute(k_kspace2_batch<TILD_KSPACE2_NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-#endif
 }
 #if TILD_KSPACE2_NF <= 2   // a batch's replicas have one or two density fields
+template <>
+void kspace2_batch_attributes<TILD_KSPACE2_NF>(int smem)
+{
+    cudaFuncSetAttribute(k_kspace2_batch<TILD_KSPACE2_NF>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+}
 template <>
 cudaError_t kspace2_launch_batch<TILD_KSPACE2_NF>(const BatchRep *reps, int R, const BatchLaunch &bl, cudaStream_t st)
 {

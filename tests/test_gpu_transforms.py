@@ -1,0 +1,94 @@
+"""Transform passes of two register stages and the int32 deposits, at the sizes where they can
+go wrong, against the FP64 oracle.
+
+Tolerances: forces max_p |df_p| / max(|f_p|, f_rms) <= 1e-5 and pair energies 1e-5 relative
+(FP32 deposit, transforms of at most 256 points per axis and gather: a few hundred roundings of
+6e-8, added in quadrature); deterministic deposits are exact integer sums, so results that
+differ only in how a tile is summed are equal bit for bit.
+"""
+import numpy as np
+import pytest
+
+import oracle
+import tild_b200
+from conftest import force_error, spec_to_system
+from tild_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def make_box(spec, **opts):
+    o = {"write_files": 0}
+    o.update(opts)
+    b = tild_b200.box_from_spec(spec, options=o)
+    b.command("endBox")
+    return b
+
+
+def species_system(nsp, grid, seed=5):
+    """Short chains of nsp species with every pair interacting: nsp density fields and force groups."""
+    rng = np.random.default_rng(seed)
+    L = np.array([0.45 * g for g in grid])
+    x = synth.random_walk_chains(rng, 60, 6, L, 0.6)
+    types = rng.integers(0, nsp, size=len(x)).astype(np.int32)
+    names = ["A", "B", "C", "D"][:nsp]
+    pots = [dict(kind="gaussian", I=a, J=b, A=1.0 + 0.3 * i + 0.2 * j, sigma=0.7)
+            for i, a in enumerate(names) for j, b in enumerate(names) if i <= j]
+    return synth.SystemSpec("species", L, grid, x, types, names, synth.chain_bonds(60, 6), np.repeat(np.arange(60), 6),
+                            potentials=pots, order=3, seed=seed)
+
+
+# every radix from 1 to 16 in either stage; one-stage lines (5, 7, 11, 13), the longest (256,
+# 240, 225, 208), and axes that keep the mixed-radix path (17, 34, 250) beside ones that do not
+@pytest.mark.parametrize("grid", [(6, 8, 9), (5, 7, 11), (13, 10, 12), (14, 15, 16), (22, 26, 33), (49, 18, 20), (64, 9, 8),
+                                  (256, 8, 6), (8, 240, 6), (6, 8, 225), (208, 7, 6), (17, 16, 12), (16, 34, 12), (12, 8, 250)])
+@pytest.mark.parametrize("nsp", [1, 2, 3, 4])
+def test_transforms_match_oracle(grid, nsp):
+    if nsp > 2 and max(grid) > 100:
+        pytest.skip("field counts are covered on the smaller grids")
+    spec = species_system(nsp, grid)
+    sysm = spec_to_system(spec)
+    fref, inter = oracle.forces(sysm, prec=64)
+    eref = np.array(oracle.pair_energies(sysm, inter["dens"]))
+    with make_box(spec) as b:
+        assert force_error(b.forces(), fref) <= 1e-5
+        e = np.array(b.thermo()["potentials"])
+        assert np.all(np.abs(e - eref) <= 1e-5 * np.abs(eref).max())
+        k, s, n = b.structure_factor("A", 8, 5.0)
+        kr, sr, nr = oracle.structure_factor(sysm, inter["dens"]["A"][0], 8, 5.0)
+        assert np.array_equal(n, nr) and np.allclose(s, sr, rtol=1e-4, atol=1e-9)
+
+
+@pytest.mark.parametrize("charge", [1.0, 0.5, 2.5])
+@pytest.mark.parametrize("deterministic", [0, 1])
+def test_deposit_coefficients_match_oracle(charge, deterministic):
+    # charges of +-1 (one conversion for both fields), other magnitudes (one each), and zero
+    spec = synth.small_system(seed=31, charges=True, n_free=200)
+    spec.charges = (spec.charges * np.float32(charge)).astype(np.float32)
+    spec.potentials = [dict(kind="gaussian", I="all", J="all", A=1.5, sigma=0.7), dict(kind="charges", lB=1.0, sigma=0.5)]
+    fref, _ = oracle.forces(spec_to_system(spec), prec=64)
+    with make_box(spec, deterministic=deterministic) as b:
+        assert force_error(b.forces(), fref) <= 1e-5
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_deterministic_sums_do_not_depend_on_the_tile(order):
+    # 80,000 particles on 16^3: tiles of 8 bricks hold 10,000 (two int32 words per point), of
+    # 32 bricks 40,000 (past the bound of the words: 64-bit box), of 64 do not fit (global)
+    rng = np.random.default_rng(order)
+    n, L = 80000, 7.0
+    x = rng.uniform(0.0, L, size=(n, 3))
+    types = rng.integers(0, 2, size=n)
+    pots = [dict(kind="gaussian", I="A", J="A", A=0.01, sigma=0.7), dict(kind="gaussian", I="A", J="B", A=0.02, sigma=0.7)]
+    spec = synth.SystemSpec("dense", [L] * 3, [16] * 3, x, types, ["A", "B"], [], np.arange(n), potentials=pots, order=order)
+    out = []
+    for codes in (8, 32, 64):
+        with make_box(spec, deterministic=1, deposit_codes=codes) as b:
+            out.append(b.forces())
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+    # against the oracle for the continuous splines only: the order-4 weights (s^4 for s^3) jump
+    # at cell edges by up to 1e-2, and of 240,000 uniform coordinates some lie within FP32
+    # rounding (about 1e-6 of a cell) of an edge and fall in the other cell there
+    if order < 4:
+        fref, _ = oracle.forces(spec_to_system(spec), prec=64)
+        assert force_error(out[0], fref) <= 1e-5
