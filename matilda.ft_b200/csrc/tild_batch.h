@@ -5,12 +5,12 @@
 // A batch holds boxes (endBox processed) that share the kernels' compile-time settings:
 // 3-D, the same spline order, one or two density fields, one or two force groups, the
 // same deterministic mode, the tile gather over paired records.  Their sizes, grids,
-// potentials, tiles and integrators may all differ.  Every step stage -- the
-// deposit, the five transform passes, the tile gather, the integrator
-// pass, the step counters -- is ONE launch (a transform pass two, where only some replicas'
-// lines run in two register stages) whose CTAs are dealt over the replicas' work by
-// a prefix table of CTA counts; each replica's geometry, FFT plans, tile lists, record
-// layout, TMA descriptors and arrays sit in a device table.  The launches of a step are
+// potentials, tiles and integrators may all differ.  Every step stage -- the deposit, the
+// five transform passes, the tile gather, the integrator pass, the step counters -- is ONE
+// launch (a transform pass two, where only some replicas' lines run in two register stages)
+// whose CTAs are dealt over the replicas' work by a prefix table of CTA counts; each
+// replica's geometry, FFT plans, tile lists, record layout, TMA descriptors and arrays sit in
+// a device table.  The launches of a step are
 // captured once in a CUDA graph.  Every sort_interval steps each replica's spatial re-sort
 // runs as a branch of one more graph.
 //
