@@ -289,6 +289,14 @@ inline bool fft_two_stage(const FftLine &lx, const FftLine &ly, const FftLine &l
 {
     return lx.r1 > 0 && ly.r1 > 0 && lz.r1 > 0 && nd == nfg && nd >= 1 && nd <= 4;
 }
+// Whether the two-stage y pass serves a field on its own (a structure factor's, whatever the
+// other axes' lines): its column indices below nz hp are divided by hp with one multiplication,
+// exact only while index x (m hp - 2^32) < 2^32, m = ceil(2^32 / hp).  Every box of three
+// two-stage axes is far inside (256 x 132 x 132); nx = 3438, nz = 1500 is not.
+inline bool fft2_columns(const Geom &g, const FftLine &ly)
+{
+    return ly.r1 > 0 && (long long)g.nz * g.hp * g.hp < (1ll << 32);
+}
 cudaError_t launch_xfwd2(const Geom &g, const FftLine &lx, int nd, float2 *dep, unsigned long long *dep_fixed, float2 *H,
                          cudaStream_t st);
 // n density fields forward, n force groups inverse

@@ -921,7 +921,7 @@ cudaError_t launch_structure_factor(const Geom &g, const FftLine &lx, const FftL
                                    double dk, double *bins, cudaStream_t st)
 {
     cudaError_t e = lx.r1 ? launch_xfwd2(g, lx, 1, rho_pair, nullptr, Hs, st) : launch_xfwd(g, lx, 1, 1, rho_pair, nullptr, Hs, st);
-    if (e == cudaSuccess) e = ly.r1 ? launch_ypass2(g, ly, 1, 0, Hs, st) : launch_ypass(g, ly, 1, 0, Hs, st);
+    if (e == cudaSuccess) e = fft2_columns(g, ly) ? launch_ypass2(g, ly, 1, 0, Hs, st) : launch_ypass(g, ly, 1, 0, Hs, st);
     if (e != cudaSuccess) return e;
     constexpr int TX = kTXz;
     dim3 grid((g.nxh + TX - 1) / TX, g.ny);

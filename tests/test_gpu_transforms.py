@@ -92,3 +92,20 @@ def test_deterministic_sums_do_not_depend_on_the_tile(order):
     if order < 4:
         fref, _ = oracle.forces(spec_to_system(spec), prec=64)
         assert force_error(out[0], fref) <= 1e-5
+
+
+def test_structure_factor_of_long_x_and_z_lines():
+    # x and z far past the two-stage lengths beside a y axis of 4 = 2 x 2: nz hp^2 >= 2^32, past
+    # the two-stage y pass's column division.  Spacings of 20 in y and z put the columns of the
+    # x Nyquist index, the last of a row, in shells of their own.
+    grid, L = [3910, 4, 1200], [0.4 * 3910, 20.0 * 4, 20.0 * 1200]
+    rng = np.random.default_rng(3)
+    n = 3000
+    x = rng.uniform(0.0, 1.0, size=(n, 3)) * L
+    spec = synth.SystemSpec("rod", L, grid, x, np.zeros(n, np.int32), ["A"], [], np.arange(n),
+                            potentials=[dict(kind="gaussian", I="A", J="A", A=0.1, sigma=0.7)], order=1)
+    with make_box(spec, sort_interval=0) as b:
+        rho = b.density("A")
+        k, s, c = b.structure_factor("A", 1963, 7.87)
+    kr, sr, cr = oracle.structure_factor(spec_to_system(spec), rho, 1963, 7.87)
+    assert np.array_equal(c, cr) and np.allclose(k, kr, rtol=1e-9) and np.allclose(s, sr, rtol=1e-4, atol=0.0)
