@@ -252,7 +252,9 @@ void Batch::buildGroup(Group &G)
     const cudaStream_t st = G.stream;
     cudaGraph_t gr;
     batch_ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
-    cudaError_t e = launch_deposit_batch(G.dReps, R, G.launches[BS_DEPOSIT], order, nd, deterministic, st);
+    int halves = 0;
+    for (const BatchRep &e : h) halves |= e.dtiles.halves;
+    cudaError_t e = launch_deposit_batch(G.dReps, R, G.launches[BS_DEPOSIT], order, nd, deterministic, halves, st);
     for (int s : {BS_XFWD, BS_YFWD, BS_KSPACE, BS_YINV, BS_XINV})
     {
         if (e == cudaSuccess && G.launches[s].blocks)

@@ -1272,16 +1272,20 @@ void Box::allocDevice()
         tiles = tileGeometry(codes, directGather);
         dtiles = tileGeometry(depositCodes ? depositCodes : codes, true);
         // The deposit's own tiles: 16 bricks and CTAs of 128 threads zero and flush a third fewer
-        // halo points per particle than 8 (1,048,576 particles on 160^3: 92 -> 72 us, 2,097,152
-        // on 192^3: 205 -> 175), where the GPU still gets four CTAs per SM of them (429 tiles
-        // of a 75^3 box: 25.0 -> 26.4 us) and the tiles' counts stay within the finest
-        // fixed-point scale (mean plus four standard deviations)
+        // halo points per particle than 8 (1,048,576 particles on 160^3: 92 -> 73 us, 2,097,152
+        // on 192^3: 205 -> 176), where the GPU still gets four CTAs per SM of them (429 tiles
+        // of a 75^3 box: 25.0 -> 26.4 us) and few tiles pass the count of the finest
+        // fixed-point scale (a Poisson mean plus four standard deviations).  Chains spread about
+        // three times as far: 32 of the 4,000 tiles of the unrelaxed 160^3 melt pass it.  Such
+        // tiles are summed in halves of 8 bricks (82 us there), so that no sum has fewer bits
+        // than with tiles of 8.
         const double e16 = 16.0 * 64.0 * (double)N / (double)g.M;
         const long long tiles16 = (long long)((g.nx + 15) / 16) * ((g.ny + 7) / 8) * ((g.nz + 7) / 8);
-        if (!depositCodes && !depositThreads && !deterministic && nd <= 2 && codes < 16 && g.nz >= 4 &&
+        if (!depositCodes && !depositThreads && !deterministic && nd <= 2 && codes == 8 && g.nz >= 4 &&
             tiles16 >= 4 * 148 && e16 + 4.0 * std::sqrt(e16) <= ppHost.int_tile_max) {
             dtiles = tileGeometry(16, true);
             dtiles.threads = 128;
+            dtiles.halves = 1;
         }
         attachTileList(tiles);
         attachTileList(dtiles);

@@ -161,6 +161,7 @@ struct TileCfg {
     int nlist;
     int nkeys;
     int codes;
+    int halves;   // deposit: 1 = tiles past the finest fixed-point scale's count go in two halves (deposit_tile)
     int threads;
     int box;      // deposit: shared-memory records of a tile's bounding box (estimate)
     int pbox;     // particle pass: records of the fixed tile box (odd pitches)
@@ -249,7 +250,7 @@ cudaError_t launch_batch_tick(const BatchRep *reps, int R, cudaStream_t st);
 // per-file pieces of the above (tild_grid.cu, tild_fft.cu, tild_particles.cu)
 void deposit_batch_shape(const BatchRep &r, int deterministic, int *blocks, int *threads, size_t *smem, int *cap);
 cudaError_t launch_deposit_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int order, int nd,
-                                 int deterministic, cudaStream_t st);
+                                 int deterministic, int halves, cudaStream_t st);   // halves: some replica's tiles have them
 int fft_batch_lines(int stage, const Geom &g, int nfg);   // lines per block of the x passes
 void fft_batch_shape(int stage, const BatchRep &r, int *blocks, int *threads, size_t *smem);
 cudaError_t launch_fft_batch(int stage, const BatchRep *reps, int R, const BatchLaunch &bl, int deterministic, int txz,

@@ -227,14 +227,14 @@ __device__ __forceinline__ void deposit_points(int *b0, int *b1, int E0, int E01
         }
 }
 
-// Deposit of one tile of sorted particles (or a window of slots).  The box of grid points
-// is accumulated in shared memory, each thread adding its particle's (P+1)^3 points with
-// shared-memory atomics (the atomics have throughput to spare; what bounds the deposit
+// Deposit of the slots [b0, b1) of one tile of sorted particles (or of a window).  The box of
+// grid points is accumulated in shared memory, each thread adding its particle's (P+1)^3 points
+// with shared-memory atomics (the atomics have throughput to spare; what bounds the deposit
 // is instruction issue, so a particle's stencil is computed once, by its own thread, and
 // converted to fixed point once per point).  Each touched point is flushed once.
 // NF: number of density fields when 1 or 2 (unrolled), 0 = any.
 template <int P, int NF, bool FIXED>
-__device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, int nd, unsigned dq,
+__device__ __forceinline__ void deposit_body(const Geom &g, int b0, int b1, int quirk4, int nd, unsigned dq,
                                              const float *__restrict__ X0, const float *__restrict__ X1,
                                              const long long *__restrict__ d_step,
                                              const uint32_t *__restrict__ pflags,
@@ -247,9 +247,6 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ TileShared ts;
     const float *__restrict__ X = (*d_step & 1) ? X1 : X0;
-    int b0, b1;
-    tile_range(tc, N, kDepPB, b0, b1, bx);
-    if (b1 <= b0) return;
     const int nn[3] = {g.nx, g.ny, g.nz};
     // sorted tiles: the fixed box of the tile's bricks plus the drift margin; particles
     // whose stencil left it deposit with global atomics (windows of unsorted slots: all)
@@ -472,7 +469,30 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int N, int quirk4, i
     });
 }
 
-template <int P, int NF, bool FIXED>
+// Deposit of CTA bx's tile or window.  HV: where the tiles ask for it (tc.halves), a tile of more
+// particles than the finest fixed-point scale takes goes in two halves of its bricks, each at the
+// scale of its own count.  call(b0, b1) deposits a range of slots.
+template <bool HV, typename F>
+__device__ __forceinline__ void deposit_tile(const TileCfg &tc, int N, int int_tile_max, unsigned bx, F call)
+{
+    int b0, b1;
+    tile_range(tc, N, kDepPB, b0, b1, bx);
+    if (!HV) {
+        if (b1 > b0) call(b0, b1);
+        return;
+    }
+    const int end = b1;
+    if (tc.halves && b1 - b0 > int_tile_max) b1 = (int)tc.start[tile_id(tc, bx) * tc.codes + tc.codes / 2];
+#pragma unroll 1
+    while (b0 < end) {
+        if (b1 > b0) call(b0, b1);
+        b0 = b1;
+        b1 = end;
+        if (b0 < end) __syncthreads();   // the first half's box is flushed
+    }
+}
+
+template <int P, int NF, bool FIXED, bool HV>
 __global__ void __launch_bounds__(512) k_deposit_tiled(Geom g, int N, int quirk4, int nd, unsigned dq,
                                                        const float *__restrict__ X0, const float *__restrict__ X1,
                                                        const long long *__restrict__ d_step,
@@ -481,19 +501,28 @@ __global__ void __launch_bounds__(512) k_deposit_tiled(Geom g, int N, int quirk4
                                                        unsigned long long *__restrict__ depfix, int cap_bytes,
                                                        TileCfg tc, int int_tile_max)
 {
-    deposit_body<P, NF, FIXED>(g, N, quirk4, nd, dq, X0, X1, d_step, pflags, q, dep, depfix, cap_bytes, tc,
-                               int_tile_max, blockIdx.x);
+    deposit_tile<HV>(tc, N, int_tile_max, blockIdx.x, [&](int b0, int b1) {
+        deposit_body<P, NF, FIXED>(g, b0, b1, quirk4, nd, dq, X0, X1, d_step, pflags, q, dep, depfix, cap_bytes, tc,
+                                   int_tile_max, blockIdx.x);
+    });
 }
 
 // the deposit over several replicas (one launch; see BatchRep)
-template <int P, int NF, bool FIXED>
+template <int P, int NF, bool FIXED, bool HV>
 __global__ void __launch_bounds__(512) k_deposit_batch(const BatchRep *__restrict__ reps, const int *__restrict__ pre,
                                                        int R)
 {
     const int r = batch_replica(pre, R, blockIdx.x);
-    const BatchRep &b = reps[r];
-    deposit_body<P, NF, FIXED>(b.g, b.N, b.quirk4, b.nd, b.dq, b.X0, b.X1, b.d_step, b.flags, b.q, b.dep, b.depfix,
-                               b.dep_cap, b.dtiles, b.int_tile_max, blockIdx.x - pre[r]);
+    const unsigned bx = blockIdx.x - pre[r];
+    deposit_tile<HV>(reps[r].dtiles, reps[r].N, reps[r].int_tile_max, bx, [&](int b0, int b1) {
+        // the pointer made anew for each call: the replica's fields, hoisted out of the loop over
+        // the halves, would hold a third of the registers
+        const BatchRep *bp = reps + r;
+        if (HV) asm volatile("" : "+l"(bp));
+        const BatchRep &b = *bp;
+        deposit_body<P, NF, FIXED>(b.g, b0, b1, b.quirk4, b.nd, b.dq, b.X0, b.X1, b.d_step, b.flags, b.q, b.dep, b.depfix,
+                                   b.dep_cap, b.dtiles, b.int_tile_max, bx);
+    });
 }
 
 // the deposit's box capacity in bytes (the host's estimate for sorted tiles, capped)
@@ -511,14 +540,13 @@ static void dep_launch_nf(int nb, int threads, const Geom &g, const ParticlePara
 {
     // box capacity: the host's estimate for sorted tiles (no staging unsorted), capped
     const int cap = deposit_cap(tc, NF ? NF : pp.nd, depfix != nullptr);
-    if (depfix)
-        k_deposit_tiled<P, NF, true><<<nb, threads, cap, st>>>(g, pp.N, pp.quirk4, pp.nd, pp.dchan_charge, X0,
-                                                                       X1, d_step, pflags, q, dep, depfix, cap, tc,
-                                                                       pp.int_tile_max);
-    else
-        k_deposit_tiled<P, NF, false><<<nb, threads, cap, st>>>(g, pp.N, pp.quirk4, pp.nd, pp.dchan_charge, X0,
-                                                                        X1, d_step, pflags, q, dep, depfix, cap, tc,
-                                                                        pp.int_tile_max);
+    auto go = [&](auto kernel) {
+        kernel<<<nb, threads, cap, st>>>(g, pp.N, pp.quirk4, pp.nd, pp.dchan_charge, X0, X1, d_step, pflags, q, dep, depfix, cap,
+                                         tc, pp.int_tile_max);
+    };
+    if (depfix) go(k_deposit_tiled<P, NF, true, false>);
+    else if (NF && tc.start && tc.halves) go(k_deposit_tiled<P, NF, false, NF != 0>);
+    else go(k_deposit_tiled<P, NF, false, false>);
 }
 
 template <int P>
@@ -545,12 +573,13 @@ void deposit_batch_shape(const BatchRep &r, int deterministic, int *blocks, int 
 }
 
 cudaError_t launch_deposit_batch(const BatchRep *reps, int R, const BatchLaunch &bl, int order, int nd,
-                                 int deterministic, cudaStream_t st)
+                                 int deterministic, int halves, cudaStream_t st)
 {
-#define TILD_DB(P, NF)                                                                                      \
-    do {                                                                                                    \
-        if (deterministic) k_deposit_batch<P, NF, true><<<bl.blocks, bl.threads, bl.smem, st>>>(reps, bl.pre, R); \
-        else k_deposit_batch<P, NF, false><<<bl.blocks, bl.threads, bl.smem, st>>>(reps, bl.pre, R);         \
+#define TILD_DB(P, NF)                                                                                             \
+    do {                                                                                                           \
+        if (deterministic) k_deposit_batch<P, NF, true, false><<<bl.blocks, bl.threads, bl.smem, st>>>(reps, bl.pre, R); \
+        else if (halves) k_deposit_batch<P, NF, false, true><<<bl.blocks, bl.threads, bl.smem, st>>>(reps, bl.pre, R);  \
+        else k_deposit_batch<P, NF, false, false><<<bl.blocks, bl.threads, bl.smem, st>>>(reps, bl.pre, R);          \
     } while (0)
 #define TILD_DBP(P) do { if (nd == 1) TILD_DB(P, 1); else TILD_DB(P, 2); } while (0)
     switch (order) {
@@ -567,12 +596,16 @@ cudaError_t launch_deposit_batch(const BatchRep *reps, int R, const BatchLaunch 
 
 void init_deposit_attributes()
 {
-#define TILD_DA1(P, NF)                                                                                        \
-    cudaFuncSetAttribute(k_deposit_tiled<P, NF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDepSmemFixed); \
-    cudaFuncSetAttribute(k_deposit_tiled<P, NF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDepSmemFast); \
-    cudaFuncSetAttribute(k_deposit_batch<P, NF, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDepSmemFixed);  \
-    cudaFuncSetAttribute(k_deposit_batch<P, NF, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kDepSmemFast)
-#define TILD_DA(P) TILD_DA1(P, 0); TILD_DA1(P, 1); TILD_DA1(P, 2)
+    auto big = [](auto *fn, int bytes) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
+#define TILD_DA1(P, NF)                                     \
+    big(k_deposit_tiled<P, NF, true, false>, kDepSmemFixed); \
+    big(k_deposit_tiled<P, NF, false, false>, kDepSmemFast); \
+    big(k_deposit_tiled<P, NF, false, NF != 0>, kDepSmemFast)
+#define TILD_DA2(P, NF)                                     \
+    big(k_deposit_batch<P, NF, true, false>, kDepSmemFixed); \
+    big(k_deposit_batch<P, NF, false, false>, kDepSmemFast); \
+    big(k_deposit_batch<P, NF, false, true>, kDepSmemFast)
+#define TILD_DA(P) TILD_DA1(P, 0); TILD_DA1(P, 1); TILD_DA1(P, 2); TILD_DA2(P, 1); TILD_DA2(P, 2)
     TILD_DA(0);
     TILD_DA(1);
     TILD_DA(2);
@@ -580,6 +613,7 @@ void init_deposit_attributes()
     TILD_DA(4);
 #undef TILD_DA
 #undef TILD_DA1
+#undef TILD_DA2
 }
 
 cudaError_t launch_deposit(const Geom &g, const ParticleParams &pp, const float *X0, const float *X1,

@@ -109,3 +109,50 @@ def test_structure_factor_of_long_x_and_z_lines():
         k, s, c = b.structure_factor("A", 1963, 7.87)
     kr, sr, cr = oracle.structure_factor(spec_to_system(spec), rho, 1963, 7.87)
     assert np.array_equal(c, cr) and np.allclose(k, kr, rtol=1e-9) and np.allclose(s, sr, rtol=1e-4, atol=0.0)
+
+
+def default_deposit_box(x, q, pots, order, **opts):
+    """A box of 88^3 points whose default deposit tiles are 16 bricks of 4^3 cells."""
+    n = len(x)
+    spec = synth.SystemSpec("tiles", [88.0] * 3, [88] * 3, x, np.zeros(n, np.int32), ["A"], [], np.arange(n), charges=q,
+                            potentials=pots, order=order)
+    b = make_box(spec, tile_codes=8, **opts)
+    t = b.describe()["tiles"]
+    assert (t["deposit_codes"], t["deposit_threads"]) == (16, 128)
+    return spec, b
+
+
+def test_dense_default_deposit_tiles_keep_the_finest_scale():
+    # Order 1: int32 sums at 2^24 per unit weight take 115 particles of charge 1.  Charges +1 at
+    # s = 1/256 and 5/256 of a cell and -1 twice at 3/256, alike in y and z: every weight is a
+    # multiple of 2^-24 and the four cancel point by point, in sums at 2^24 exactly, while at
+    # 2^23 the odd multiples round.  100 of them in each half of one 16-brick tile.
+    rng = np.random.default_rng(9)
+    x, q = [], []
+    for half in (0, 8):
+        for _ in range(25):
+            c = rng.integers(1, 7, size=3) + [half, 0, 0]
+            yz = (2 * rng.integers(-60, 60, size=2) + 1) / 256.0
+            for s, v in ((1, 1.0), (5, 1.0), (3, -1.0), (3, -1.0)):
+                x.append(c + 0.5 + np.array([s / 256.0, yz[0], yz[1]]))
+                q.append(v)
+    spec, b = default_deposit_box(np.array(x), np.array(q, np.float32), [dict(kind="charges", lB=1.0, sigma=0.5)], 1)
+    with b:
+        assert np.array_equal(b.forces(), np.zeros_like(spec.x))
+
+
+@pytest.mark.parametrize("counts", [(100, 100), (300, 40), (0, 900), (1500, 1200)])
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+def test_dense_default_deposit_tiles_match_oracle(order, counts):
+    # the halves of one tile at each fixed-point scale, empty, and past all scales (FP32)
+    rng = np.random.default_rng(sum(counts) + order)
+    x = np.concatenate([rng.uniform(0.0, 8.0, size=(n, 3)) + [8.0 * h, 0.0, 0.0] for h, n in enumerate(counts)] +
+                       [rng.uniform(0.0, 88.0, size=(500, 3))])
+    if order == 4:   # away from cell edges, where the order-4 weights jump (see above)
+        x = np.floor(x) + 0.05 + 0.9 * (x - np.floor(x))
+        x = np.where(np.abs(x - np.floor(x) - 0.5) < 0.02, x + 0.04, x)
+    spec, b = default_deposit_box(x, None, [dict(kind="gaussian", I="A", J="A", A=0.5, sigma=0.7)], order)
+    with b:
+        f = b.forces()
+    fref, _ = oracle.forces(spec_to_system(spec), prec=64)
+    assert force_error(f, fref) <= 1e-5
