@@ -251,6 +251,8 @@ void Batch::buildGroup(Group &G)
     // the step: deposit, x/y forward, k-space, y/x inverse, gather, integrate, tick
     const cudaStream_t st = G.stream;
     cudaGraph_t gr;
+    init_deposit_attributes(order, nd, deterministic, 1);
+    init_particle_attributes(order, 1);
     batch_ck(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "begin capture");
     int halves = 0;
     for (const BatchRep &e : h) halves |= e.dtiles.halves;

@@ -25,10 +25,6 @@
 
 namespace tild {
 
-void init_fft_attributes();
-void init_deposit_attributes();
-void init_particle_attributes();
-
 [[noreturn]] void fail(int code, const std::string &msg) { throw BoxError{code, msg}; }
 
 namespace {
@@ -993,8 +989,6 @@ void Box::initDevice()
         ck(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
         ownStream = true;
     }
-    init_deposit_attributes();
-    init_particle_attributes();
     allocDevice();
     uploadParticles();
     if (sortInterval > 0) {   // start from a spatially coherent order
@@ -1315,14 +1309,17 @@ void Box::allocDevice()
     sortW.ang = nAnglesTot > 0 ? dalloc<int>(3 * N * MAXANGLES) : nullptr;
 }
 
-// The transform passes this box's fields take and the blocks of its k-space pass.
+// The transform passes this box's fields take and the blocks of its k-space pass; large shared
+// memory for the kernels it launches, and for no others (each call loads its kernel).
 void Box::planTransforms()
 {
     const int nd = (int)dfields.size(), nfg = (int)fgroups.size();
     twoStage = fft_two_stage(lx, ly, lz, nd, nfg);
     nblkZ = kspace_blocks(geom, lz, nd, nfg, (int)potentials.size(), twoStage);
-    if (twoStage) init_fft2_attributes(nd);   // only the kernels this box launches: each call costs set-up time
+    if (twoStage) init_fft2_attributes(nd);
     else init_fft_attributes();
+    init_deposit_attributes(pmeorder, nd, deterministic, 0);
+    init_particle_attributes(pmeorder, 0);
 }
 
 void Box::uploadParticles()

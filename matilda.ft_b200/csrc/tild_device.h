@@ -265,7 +265,9 @@ cudaError_t launch_particles_batch(int stage, const BatchRep *reps, int R, const
 // plan of one axis: tables in dev[3n] (uploaded on st, complete on return)
 void build_fft_line(int n, double twopi_over_L, FftLine &pl, float2 *dev);
 void init_fft_attributes();      // opt the FFT kernels into large dynamic shared memory
-void init_deposit_attributes();  // same for the staged deposit
+// same for the staged deposit and the gather of boxes (or batches) of one order, field count and mode
+void init_deposit_attributes(int order, int nd, int deterministic, int batch);
+void init_particle_attributes(int order, int batch);
 cudaError_t launch_deposit(const Geom &g, const ParticleParams &pp, const float *X0,
                            const float *X1, const long long *d_step, const uint32_t *pflags,
                            const float *q, float2 *dep, unsigned long long *dep_fixed,
@@ -357,7 +359,6 @@ cudaError_t launch_integrate(const Geom &g, const ParticleParams &pp, const Part
                              cudaStream_t st);
 // whether the paired tile gather can stage a box of te[] points for nfg force groups
 bool paired_box_fits(const int *te, int nfg);
-void init_particle_attributes();
 cudaError_t launch_tick(long long *d_step, cudaStream_t st);
 
 // ---- spatial re-sort (tild_sort.cu) ----

@@ -594,26 +594,41 @@ cudaError_t launch_deposit_batch(const BatchRep *reps, int R, const BatchLaunch 
     return cudaGetLastError();
 }
 
-void init_deposit_attributes()
+// Large dynamic shared memory for the deposit kernels of boxes of this order, field count and mode
+template <int P, int NF>
+static void deposit_attributes(bool batch, bool fixed)
 {
-    auto big = [](auto *fn, int bytes) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes); };
-#define TILD_DA1(P, NF)                                     \
-    big(k_deposit_tiled<P, NF, true, false>, kDepSmemFixed); \
-    big(k_deposit_tiled<P, NF, false, false>, kDepSmemFast); \
-    big(k_deposit_tiled<P, NF, false, NF != 0>, kDepSmemFast)
-#define TILD_DA2(P, NF)                                     \
-    big(k_deposit_batch<P, NF, true, false>, kDepSmemFixed); \
-    big(k_deposit_batch<P, NF, false, false>, kDepSmemFast); \
-    big(k_deposit_batch<P, NF, false, true>, kDepSmemFast)
-#define TILD_DA(P) TILD_DA1(P, 0); TILD_DA1(P, 1); TILD_DA1(P, 2); TILD_DA2(P, 1); TILD_DA2(P, 2)
-    TILD_DA(0);
-    TILD_DA(1);
-    TILD_DA(2);
-    TILD_DA(3);
-    TILD_DA(4);
+    auto big = [&](auto *fn) {
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, fixed ? kDepSmemFixed : kDepSmemFast);
+    };
+    if constexpr (NF != 0) {
+        if (batch) {
+            if (fixed) return big(k_deposit_batch<P, NF, true, false>);
+            big(k_deposit_batch<P, NF, false, false>);
+            return big(k_deposit_batch<P, NF, false, true>);
+        }
+        if (!fixed) big(k_deposit_tiled<P, NF, false, true>);
+    }
+    if (fixed) big(k_deposit_tiled<P, NF, true, false>);
+    else big(k_deposit_tiled<P, NF, false, false>);
+}
+
+void init_deposit_attributes(int order, int nd, int deterministic, int batch)
+{
+#define TILD_DA(P)                                                               \
+    do {                                                                         \
+        if (nd == 1) deposit_attributes<P, 1>(batch != 0, deterministic != 0);   \
+        else if (nd == 2) deposit_attributes<P, 2>(batch != 0, deterministic != 0); \
+        else deposit_attributes<P, 0>(batch != 0, deterministic != 0);           \
+    } while (0)
+    switch (order) {
+        case 0: TILD_DA(0); break;
+        case 1: TILD_DA(1); break;
+        case 2: TILD_DA(2); break;
+        case 3: TILD_DA(3); break;
+        default: TILD_DA(4); break;
+    }
 #undef TILD_DA
-#undef TILD_DA1
-#undef TILD_DA2
 }
 
 cudaError_t launch_deposit(const Geom &g, const ParticleParams &pp, const float *X0, const float *X1,

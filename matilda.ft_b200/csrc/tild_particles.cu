@@ -1478,20 +1478,28 @@ bool build_paired_maps(CUtensorMap *mapA, CUtensorMap *mapB, const RecLayout &rl
            CUDA_SUCCESS;
 }
 
-void init_particle_attributes()
+void init_particle_attributes(int order, int batch)
 {
-#define TILD_PA(P)                                                                                        \
-    cudaFuncSetAttribute(k_gather_planar<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPartSmemMax); \
-    cudaFuncSetAttribute(k_gather_planar<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPartSmemMax);  \
-    cudaFuncSetAttribute(k_gather_paired<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMax);     \
-    cudaFuncSetAttribute(k_gather_paired<P, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMax);     \
-    cudaFuncSetAttribute(k_gather_batch<P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMax);      \
-    cudaFuncSetAttribute(k_gather_batch<P, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmemMax)
-    TILD_PA(0);
-    TILD_PA(1);
-    TILD_PA(2);
-    TILD_PA(3);
-    TILD_PA(4);
+    auto big = [](auto *fn, size_t bytes) { cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+#define TILD_PA(P)                                      \
+    do {                                                \
+        if (batch) {                                    \
+            big(k_gather_batch<P, 1>, kPairSmemMax);    \
+            big(k_gather_batch<P, 2>, kPairSmemMax);    \
+        } else {                                        \
+            big(k_gather_planar<P, false>, kPartSmemMax); \
+            big(k_gather_planar<P, true>, kPartSmemMax);  \
+            big(k_gather_paired<P, 1>, kPairSmemMax);   \
+            big(k_gather_paired<P, 2>, kPairSmemMax);   \
+        }                                               \
+    } while (0)
+    switch (order) {
+        case 0: TILD_PA(0); break;
+        case 1: TILD_PA(1); break;
+        case 2: TILD_PA(2); break;
+        case 3: TILD_PA(3); break;
+        default: TILD_PA(4); break;
+    }
 #undef TILD_PA
 }
 

@@ -156,3 +156,38 @@ def test_dense_default_deposit_tiles_match_oracle(order, counts):
         f = b.forces()
     fref, _ = oracle.forces(spec_to_system(spec), prec=64)
     assert force_error(f, fref) <= 1e-5
+
+
+@pytest.mark.parametrize("order", [1, 2, 3, 4])
+@pytest.mark.parametrize("nsp,deterministic", [(1, 1), (2, 0), (3, 0), (3, 1)])
+def test_large_deposit_boxes_launch_for_each_kernel(order, nsp, deterministic):
+    # deposit tiles of 64 bricks (16 for three fields in 64 bits): boxes past the 48 KB that a
+    # kernel has without opting in, alone, in a batch, and after the field count has dropped
+    spec = species_system(nsp, (32, 32, 32), seed=order)
+    spec.order = order
+    if order == 4:   # away from cell edges, where the order-4 weights jump (see above)
+        h = spec.L[0] / 32
+        c = np.floor(spec.x / h)
+        spec.x = ((c + 0.1 + 0.3 * (spec.x / h - c)) * h).astype(np.float32)
+    opts = dict(deterministic=deterministic, tile_codes=8, deposit_codes=16 if nsp == 3 and deterministic else 64)
+    fref, _ = oracle.forces(spec_to_system(spec), prec=64)
+    with make_box(spec, **opts) as b:
+        assert force_error(b.forces(), fref) <= 1e-5
+        if nsp > 1:
+            for _ in range(nsp):   # the interactions of the first species: one field fewer
+                b.modify("potential remove 1")
+            rest = list(spec.potentials)[nsp:]
+            sub, _ = oracle.forces(spec_to_system(synth.SystemSpec(
+                "rest", spec.L, spec.grid, spec.x, spec.types, spec.species, spec.bonds, spec.mol, potentials=rest,
+                order=order)), prec=64)
+            assert force_error(b.forces(), sub) <= 1e-5
+    if nsp < 3:
+        with make_box(spec, **opts) as b:
+            b.step(2)
+            alone = b.positions()
+        with make_box(spec, **opts) as b, tild_b200.Batch() as batch:
+            batch.add(b)
+            batch.step(2)
+            d = b.positions() - alone
+            batch.close()
+        assert np.abs(d - np.round(d / spec.L) * spec.L).max() <= (0.0 if deterministic else 1e-3)
