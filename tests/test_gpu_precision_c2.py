@@ -29,15 +29,19 @@ def c2_reference():
     return spec, sysm, fref, inter
 
 
-# the density rule's deposit tiles (8 bricks: int32 boxes at 2^24 per unit weight), and the
-# 32- and 64-brick tiles the autotuner picks on this workload (about 600 and 1,200 particles
-# each: 2^23 and 2^22, FP32 for the rare tile past four times the count bound)
-@pytest.mark.parametrize("deposit_codes,deposit_threads", [(0, 0), (32, 0), (64, 512)])
+# the default deposit tiles (16 bricks, dense ones in halves: int32 boxes at 2^24 per unit weight),
+# tiles of the particle pass's 8 bricks, and the 32- and 64-brick tiles the autotuner picks on this
+# workload (about 600 and 1,200 particles each: 2^23 and 2^22, FP32 for the rare tile past four
+# times the count bound)
+@pytest.mark.parametrize("deposit_codes,deposit_threads", [(0, 0), (8, 0), (32, 0), (64, 512)])
 def test_c2_forces_and_energies_match_the_fp64_oracle(c2_reference, deposit_codes, deposit_threads):
     spec, sysm, fref, inter = c2_reference
     opts = {"write_files": 0, "deposit_codes": deposit_codes, "deposit_threads": deposit_threads}
     with tild_b200.box_from_spec(spec, options=opts) as b:
         b.command("endBox")
+        tiles = b.describe()["tiles"]
+        assert tiles["deposit_codes"] == (deposit_codes or 16)
+        assert deposit_codes or tiles["deposit_threads"] == 128
         f = b.forces()
         th = b.thermo()
     mag = np.linalg.norm(fref, axis=1)

@@ -38,8 +38,8 @@ def species_system(nsp, grid, seed=5):
                             potentials=pots, order=3, seed=seed)
 
 
-# every radix from 1 to 16 in either stage; one-stage lines (5, 7, 11, 13), the longest (256,
-# 240, 225, 208), and axes that keep the mixed-radix path (17, 34, 250) beside ones that do not
+# one-stage lines (5, 7, 11, 13), uneven factors, the longest lines (256, 240, 225, 208), and axes
+# that keep the mixed-radix path (17, 34, 250) beside ones that do not
 @pytest.mark.parametrize("grid", [(6, 8, 9), (5, 7, 11), (13, 10, 12), (14, 15, 16), (22, 26, 33), (49, 18, 20), (64, 9, 8),
                                   (256, 8, 6), (8, 240, 6), (6, 8, 225), (208, 7, 6), (17, 16, 12), (16, 34, 12), (12, 8, 250)])
 @pytest.mark.parametrize("nsp", [1, 2, 3, 4])
@@ -57,6 +57,34 @@ def test_transforms_match_oracle(grid, nsp):
         k, s, n = b.structure_factor("A", 8, 5.0)
         kr, sr, nr = oracle.structure_factor(sysm, inter["dens"]["A"][0], 8, 5.0)
         assert np.array_equal(n, nr) and np.allclose(s, sr, rtol=1e-4, atol=1e-9)
+
+
+# every radix of either stage along every axis: k x k points for k = 3 .. 16, 3 x 2, 5 x 1, and
+# 2 x 2 (of the order-2 box)
+EDGES = [4, 5, 6, 9, 16, 25, 36, 49, 64, 81, 100, 121, 144, 169, 196, 225, 256]
+
+
+def two_stage_factors(n):
+    r1 = next(r for r in range(1, 17) if r * r >= n and n % r == 0)
+    return r1, n // r1
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("nsp", [1, 2, 3, 4])
+def test_every_radix_of_both_stages_matches_oracle(axis, nsp):
+    factors = [two_stage_factors(n) for n in EDGES]
+    assert {a for a, _ in factors} == set(range(2, 17)) and {b for _, b in factors} == set(range(1, 17))
+    for n in EDGES:
+        grid = [6, 8]
+        grid.insert(axis, n)
+        spec = species_system(nsp, tuple(grid), seed=n)
+        spec.order = 2 if n == 4 else 3
+        sysm = spec_to_system(spec)
+        fref, inter = oracle.forces(sysm, prec=64)
+        eref = np.array(oracle.pair_energies(sysm, inter["dens"]))
+        with make_box(spec) as b:
+            assert force_error(b.forces(), fref) <= 1e-5, n
+            assert np.all(np.abs(np.array(b.thermo()["potentials"]) - eref) <= 1e-5 * np.abs(eref).max()), n
 
 
 @pytest.mark.parametrize("charge", [1.0, 0.5, 2.5])
@@ -191,3 +219,44 @@ def test_large_deposit_boxes_launch_for_each_kernel(order, nsp, deterministic):
             d = b.positions() - alone
             batch.close()
         assert np.abs(d - np.round(d / spec.L) * spec.L).max() <= (0.0 if deterministic else 1e-3)
+
+
+@pytest.mark.parametrize("n,codes", [(80, 8), (88, 16)])
+def test_default_deposit_tiles_on_either_side_of_the_tile_count(n, codes):
+    # 500 and 726 tiles of 16 bricks: below and above four CTAs per SM
+    rng = np.random.default_rng(n)
+    spec = synth.SystemSpec("t", [float(n)] * 3, [n] * 3, rng.uniform(0.0, n, size=(1000, 3)), np.zeros(1000, np.int32), ["A"],
+                            [], np.arange(1000), potentials=[dict(kind="gaussian", I="A", J="A", A=0.5, sigma=0.7)], order=3)
+    with make_box(spec, tile_codes=8) as b:
+        assert b.describe()["tiles"]["deposit_codes"] == codes
+    with make_box(spec, tile_codes=8, deterministic=1) as b:
+        assert b.describe()["tiles"]["deposit_codes"] == 8
+
+
+def test_batch_of_two_stage_and_mixed_radix_boxes_with_dense_tiles():
+    # a replica whose default 16-brick tiles are dense (halves), one of two-stage lines on
+    # smaller tiles, and one on the mixed-radix path, two force groups each, in fast mode: the
+    # same kernels as alone, sums in another order (FP32 rounding carried through five steps)
+    rng = np.random.default_rng(17)
+    pots = [dict(kind="gaussian", I=a, J=c, A=v, sigma=0.7) for a, c, v in (("A", "A", 1.0), ("A", "B", 1.5), ("B", "B", 1.0))]
+    specs = []
+    for g, dense in ((88, 700), (32, 0), (34, 0)):
+        x = np.concatenate([rng.uniform(0.0, 8.0, size=(dense, 3)), rng.uniform(0.0, g, size=(2000, 3))])
+        m = len(x)
+        specs.append(synth.SystemSpec("b%d" % g, [float(g)] * 3, [g] * 3, x, np.arange(m) % 2, ["A", "B"], [], np.arange(m),
+                                      potentials=pots, order=3, seed=g))
+    alone = []
+    for s in specs:
+        with make_box(s, tile_codes=8) as b:
+            b.step(5)
+            alone.append(b.positions())
+    boxes = [make_box(s, tile_codes=8) for s in specs]
+    assert [b.describe()["tiles"]["deposit_codes"] for b in boxes] == [16, 8, 8]
+    with tild_b200.Batch() as batch:
+        for b in boxes:
+            batch.add(b)
+        batch.step(5)
+    for b, x, s in zip(boxes, alone, specs):
+        d = b.positions() - x
+        assert np.abs(d - np.round(d / s.L) * s.L).max() <= 1e-4
+        b.close()
