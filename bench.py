@@ -430,8 +430,8 @@ def run_batched(tild_b200, synth, args):
             "value": work / batch_s, "unit": METRIC, "plain_value": work / plain_s,
             "pool_value": work / pool_s, "speedup_vs_plain": plain_s / batch_s, "batched_s": batch_s,
             "plain_s": plain_s, "pool_s": pool_s,
-            "form": "tild_batch: one kernel launch per step stage over all replicas (10 per step, one CUDA "
-                    "graph); re-sorts every 10 steps as branches of one graph",
+            "form": "tild_batch: one kernel launch per step stage over all replicas (9 per step, and 5 more where grids "
+                    "run in both transform forms, one CUDA graph); re-sorts every 10 steps as branches of one graph",
             "timing": "wall clock, host, includes allocation, upload, first sort, graph capture and result copies"}
 
 

@@ -128,9 +128,11 @@ int tild_box_set_angles(tild_box *box, int64_t nangles, const int64_t *triples, 
  *                    staging its tile's box in shared memory (default 0; same bits)
  *   "tile_codes"     fixed bricks per particle tile, a power of two <= 64 (0 = from the
  *                    particle density)
- *   "deposit_codes"  fixed bricks per deposit tile, a power of two in [8, 64] (0 = chosen)
- *   "deposit_threads" fixed deposit CTA size, a multiple of 32 in [64, 512] (0 = one
- *                    thread per particle of a typical tile)
+ *   "deposit_codes"  fixed bricks per deposit tile, a power of two in [8, 64] (0 = those of
+ *                    the particle tiles, or 16 where these are 8 in a large 3-D box of one
+ *                    or two density fields in fast mode, "deposit_threads" being 0)
+ *   "deposit_threads" fixed deposit CTA size, a multiple of 32 in [64, 512] (0 = about one
+ *                    thread per particle of a typical tile, 128 for the 16-brick default)
  *   "gather_threads" fixed CTA size of the particle gather, a multiple of 32 in [64, 448]
  *                    (0 = about one thread per particle of a typical tile; same bits)
  * Must precede endBox except "write_files", "echo", "stage_timing" and "sort_interval". */
@@ -198,8 +200,9 @@ int tild_box_get_grid_force(tild_box *box, const char *group, float *gf_out);
  * allocate device memory: a host program whose pool allocator has reserved the device's
  * memory up front (so cudaMalloc fails or fragments the pool), or one that reads
  * densities between steps of other work on other streams, where cudaFree would
- * synchronise the whole device.  The device scratch (4 bytes per grid point, per
- * particle and per site of the group) comes instead from one static device array of
+ * synchronise the whole device.  (tild_box_get_density allocates nothing either: its
+ * scratch is the box's own step scratch.)  The device scratch (4 bytes per grid point, per
+ * particle and per site of the group) comes here from one static device array of
  * TILD_NOALLOC_SCRATCH_BYTES (16 MiB), which every GPU that loads the library holds until
  * the process exits.  A box needing more is refused with TILD_ERR_ARG ("... the static
  * scratch holds ...").  The first call on a device looks the array's address up

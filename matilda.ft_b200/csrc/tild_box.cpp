@@ -2394,7 +2394,7 @@ void Box::getGridForce(const std::string &group, float *gf)
     }
 }
 
-// getDensity without any allocation: the accumulator rho[M], the slot-of-particle table
+// getDensity without the box's scratch: the accumulator rho[M], the slot-of-particle table
 // slot_of[N] and the group's sites[ns] live in the static device scratch, in that order.
 // rho must start at zero and is cleared here on every call; slot_of and sites are fully
 // overwritten.  Calls on one device share the scratch and must not overlap.
@@ -2444,8 +2444,8 @@ void Box::structureFactor(const std::string &group, int charge, int nbins, doubl
         binCap = cap;
     }
     float *dRho = groupDensity(gi, charge);
-    // the packed pairs after the density in the gradient half spectra (M/2 + 2 + M complex
-    // values of at least 1.5 M + 3 ny nz), the spectrum in the density half spectra
+    // the packed pairs after the density in the gradient half spectra (at most 1.5 M + 1.5 complex
+    // values of 3 hp ny nz >= 1.5 M + 1.5 ny nz), the spectrum in the density half spectra
     float2 *dPair = dHg + ((g.M + 3) / 4) * 2;
     ck(cudaMemsetAsync(dBins, 0, 3 * sizeof(double) * nbins, stream), "clear bins");
     ck(launch_to_pairs(dRho, dPair, g.M, stream), "structure factor");

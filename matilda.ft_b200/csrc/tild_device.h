@@ -262,7 +262,7 @@ cudaError_t launch_particles_batch(int stage, const BatchRep *reps, int R, const
 // -------------------------------------------------------------------------------------
 // Launchers (tild_grid.cu, tild_fft.cu, tild_particles.cu, tild_sort.cu).  All run on `st`;
 // none synchronises.
-// plan of one axis: tables in dev[3n] (uploaded on st, complete on return)
+// plan of one axis: tables in dev[3n], uploaded by a blocking copy
 void build_fft_line(int n, double twopi_over_L, FftLine &pl, float2 *dev);
 void init_fft_attributes();      // opt the FFT kernels into large dynamic shared memory
 // same for the staged deposit and the gather of boxes (or batches) of one order, field count and mode

@@ -52,8 +52,9 @@ __device__ __forceinline__ void fft_stage(const float2 *__restrict__ src, float2
     }
 }
 
-// Generic radix stage, R an odd prime (17, 19, ...: the plan takes 2, 3, 5 and 7 first, and the
-// smaller primes of short lines run in two register stages).  With the twiddled inputs a_s,
+// Generic radix stage, R an odd prime (11, 13, 17, ...: the plan takes 2, 3, 5 and 7 first; a box
+// whose three axes all split into r1 r2 <= 16 x 16 runs in two register stages instead, but one
+// axis that does not sends the others, 11s and 13s among them, here).  With the twiddled inputs a_s,
 // t_s = a_s + a_{R-s} and u_s = a_s - a_{R-s} (s <= (R-1)/2), the output pair (q, R - q) is
 // m_q -+ i n_q with m_q = a_0 + sum_s cos(2 pi q s/R) t_s and n_q = sum_s sin(2 pi q s/R) u_s.
 // A first sweep leaves t_s and u_s in the places of a_s and a_{R-s}; then one thread per output

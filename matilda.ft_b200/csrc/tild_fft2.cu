@@ -407,7 +407,7 @@ __global__ void __maxnreg__(96) k_xinv2_batch(const BatchRep *__restrict__ reps,
 // a block of 112 threads or more (r1 >= 14), since several small blocks per SM overlap their
 // loads and transforms better than two large ones (x inverse, 8 against 16 lines: 192 points
 // 149 and 157 us, 160 points 98 and 110, 75 points 19 and 26; but 100 points, of r1 = 10, 37
-// and 30), else as the columns.
+// and 30; lengths of r1 from 11 to 13 were not compared), else as the columns.
 static int lines_of(const FftLine &l, long long nlines, int jobs, bool rows)
 {
     int L = rows && 8 * l.r1 >= 112 ? 8 : 16;

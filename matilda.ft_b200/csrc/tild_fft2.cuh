@@ -4,17 +4,16 @@
 // the thread that holds i, which transforms over q in registers (r1 points), multiplies by
 // the twiddles W_n^{i k1} and stores (k1, i); the thread that then holds k1 transforms over
 // i (r2 points) and has the outputs k1 + r1 k2.  The mixed-radix Stockham passes of
-// tild_fft.cu (lines with a prime factor above 13, or longer than 256 points) take a round
-// trip through shared memory and its index arithmetic per radix of at most 8, about 150
-// thread instructions per point for a 192-point line; here it is one round trip, loads and
-// stores go straight between global memory and registers, and a thread's index arithmetic
-// serves r1 or r2 points.
+// tild_fft.cu (boxes with an axis that has no such split: a prime factor above 13, more than
+// 256 points, or lengths like 125, 147, 162, 175, 200, 216, 243 and 250) take a round trip
+// through shared memory and its index arithmetic per radix of at most 8, about 150 thread
+// instructions per point for a 192-point line; here it is one round trip, loads and stores go
+// straight between global memory and registers, and a thread's index arithmetic serves r1 or
+// r2 points.
 #pragma once
 #include "tild_dft.cuh"
 
 namespace tild {
-
-constexpr int kRadixMax = 16;
 
 // switch over a radix known only at run time, uniform over the block
 #define TILD_RADIX(r, F)        \

@@ -4,7 +4,9 @@
 // pool allocator already holds the device's memory, or a cudaFree would synchronise
 // streams the caller keeps busy).  It needs the same device scratch as
 // tild_box_get_density (a density accumulator, a slot-of-particle table and the group's
-// site list) but takes it from one file-scope __device__ array instead of cudaMalloc.
+// site list).  That call takes it from the box's own step scratch and allocates nothing
+// either; this one takes it from one file-scope __device__ array, of a size known when
+// the library loads, whatever the box.
 // Every call on a device shares that one array and finds the previous call's contents in
 // it; calls that overlap on the same device (two boxes or two host threads) race on it.
 #include "tild_device.h"
