@@ -235,9 +235,7 @@ __device__ __forceinline__ void deposit_points(int *b0, int *b1, int E0, int E01
 // NF: number of density fields when 1 or 2 (unrolled), 0 = any.
 template <int P, int NF, bool FIXED>
 __device__ __forceinline__ void deposit_body(const Geom &g, int b0, int b1, int quirk4, int nd, unsigned dq,
-                                             const float *__restrict__ X0, const float *__restrict__ X1,
-                                             const long long *__restrict__ d_step,
-                                             const uint32_t *__restrict__ pflags,
+                                             const float *__restrict__ X, const uint32_t *__restrict__ pflags,
                                              const float *__restrict__ q, float2 *__restrict__ dep,
                                              unsigned long long *__restrict__ depfix, int cap_bytes,
                                              const TileCfg &tc, int int_tile_max, unsigned bx)
@@ -246,7 +244,6 @@ __device__ __forceinline__ void deposit_body(const Geom &g, int b0, int b1, int 
     constexpr int NC = NF ? NF : kMaxFields;
     extern __shared__ __align__(16) unsigned char smraw[];
     __shared__ TileShared ts;
-    const float *__restrict__ X = (*d_step & 1) ? X1 : X0;
     const int nn[3] = {g.nx, g.ny, g.nz};
     // sorted tiles: the fixed box of the tile's bricks plus the drift margin; particles
     // whose stencil left it deposit with global atomics (windows of unsorted slots: all)
@@ -501,9 +498,9 @@ __global__ void __launch_bounds__(512) k_deposit_tiled(Geom g, int N, int quirk4
                                                        unsigned long long *__restrict__ depfix, int cap_bytes,
                                                        TileCfg tc, int int_tile_max)
 {
+    const float *__restrict__ X = (*d_step & 1) ? X1 : X0;   // beside the loads of the tile's range
     deposit_tile<HV>(tc, N, int_tile_max, blockIdx.x, [&](int b0, int b1) {
-        deposit_body<P, NF, FIXED>(g, b0, b1, quirk4, nd, dq, X0, X1, d_step, pflags, q, dep, depfix, cap_bytes, tc,
-                                   int_tile_max, blockIdx.x);
+        deposit_body<P, NF, FIXED>(g, b0, b1, quirk4, nd, dq, X, pflags, q, dep, depfix, cap_bytes, tc, int_tile_max, blockIdx.x);
     });
 }
 
@@ -514,14 +511,15 @@ __global__ void __launch_bounds__(512) k_deposit_batch(const BatchRep *__restric
 {
     const int r = batch_replica(pre, R, blockIdx.x);
     const unsigned bx = blockIdx.x - pre[r];
+    const float *__restrict__ X = (*reps[r].d_step & 1) ? reps[r].X1 : reps[r].X0;
     deposit_tile<HV>(reps[r].dtiles, reps[r].N, reps[r].int_tile_max, bx, [&](int b0, int b1) {
-        // the pointer made anew for each call: the replica's fields, hoisted out of the loop over
-        // the halves, would hold a third of the registers
+        // the pointer made anew for each call: the replica's fields, hoisted (out of the loop over
+        // the halves, or before the tile's range), would hold a third of the registers
         const BatchRep *bp = reps + r;
-        if (HV) asm volatile("" : "+l"(bp));
+        if (!FIXED) asm volatile("" : "+l"(bp));
         const BatchRep &b = *bp;
-        deposit_body<P, NF, FIXED>(b.g, b0, b1, b.quirk4, b.nd, b.dq, b.X0, b.X1, b.d_step, b.flags, b.q, b.dep, b.depfix,
-                                   b.dep_cap, b.dtiles, b.int_tile_max, bx);
+        deposit_body<P, NF, FIXED>(b.g, b0, b1, b.quirk4, b.nd, b.dq, X, b.flags, b.q, b.dep, b.depfix, b.dep_cap, b.dtiles,
+                                   b.int_tile_max, bx);
     });
 }
 
