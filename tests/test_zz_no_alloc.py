@@ -1,9 +1,9 @@
-"""The allocation-free density read-back against the allocating one, on the GPU.
+"""The density read-back from static device scratch against the one from the box's own, on the GPU.
 
 tild_box_get_density_noalloc is for callers that cannot allocate device memory (their
 pool allocator holds the device's memory, or a cudaFree would synchronise streams they
-keep busy); it takes its device scratch from one static device array instead of
-cudaMalloc.  It must return the density tild_box_get_density returns on two calls in a
+keep busy); it takes its device scratch from one static device array, where
+tild_box_get_density takes the box's own.  It must return the density tild_box_get_density returns on two calls in a
 row (the accumulator in the static array keeps the previous call's contents, so every
 call has to clear it), and it must refuse a box whose scratch does not fit.  Tolerance:
 |drho| <= 1e-6 * max|rho| (the two entry points deposit with FP32 atomics in different
