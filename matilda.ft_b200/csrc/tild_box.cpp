@@ -1316,10 +1316,10 @@ void Box::planTransforms()
     const int nd = (int)dfields.size(), nfg = (int)fgroups.size();
     twoStage = fft_two_stage(lx, ly, lz, nd, nfg);
     nblkZ = kspace_blocks(geom, lz, nd, nfg, (int)potentials.size(), twoStage);
-    if (twoStage) init_fft2_attributes(nd);
-    else init_fft_attributes();
     init_deposit_attributes(pmeorder, nd, deterministic, 0);
     init_particle_attributes(pmeorder, 0);
+    if (twoStage) init_fft2_attributes(nd);
+    else init_fft_attributes();
 }
 
 void Box::uploadParticles()
